@@ -86,7 +86,10 @@ __global__ void __launch_bounds__(256) k_tiny(const float2* __restrict__ in, flo
     const int total = count << LOG_N;
     const float2* src = in + (first << LOG_N);
     float2* dst = out + (first << LOG_N);
-    for (int i = threadIdx.x; i < total; i += 256) s[spad(i)] = __ldg(src + i);
+    dependent_launch();
+    dependent_wait();
+    if constexpr (W) pre = after_wait(pre), post = after_wait(post);
+    for (int i = threadIdx.x; i < total; i += 256) s[spad(i)] = ld_stream(src + i);
     __syncthreads();
 #pragma unroll
     for (int p = 0; p < PER; ++p) {
@@ -169,6 +172,9 @@ __global__ void __launch_bounds__(1 << (LOG_L + LOG_C - 4))
               const float2* __restrict__ stw, const float2* __restrict__ pre, const float2* __restrict__ post) {
     extern __shared__ float2 smem[];
     const int tid = threadIdx.x;
+    dependent_launch();
+    dependent_wait();
+    if constexpr (W) pre = after_wait(pre), post = after_wait(post);
     if constexpr (LOG_L <= 6 && !W) {
         batched_tile_staged<LOG_L, LOG_C, INV>(in, out, batch, stw, smem, tid);
     } else {
@@ -181,7 +187,8 @@ __global__ void __launch_bounds__(1 << (LOG_L + LOG_C - 4))
 template <int LOG_L, int LOG_C, int MODE, bool W, bool X = false>
 __global__ void __launch_bounds__(1 << (LOG_L + LOG_C - 4)) k_pass(PassArgs a) {
     extern __shared__ float2 smem[];
-    pass_tile<LOG_L, LOG_C, MODE, 0, W, false, X>(a, blockIdx.x, X ? 0ll : (long long)blockIdx.y << a.log2n, smem,
+    dependent_launch();
+    pass_tile<LOG_L, LOG_C, MODE, 0, W, true, X>(a, blockIdx.x, X ? 0ll : (long long)blockIdx.y << a.log2n, smem,
                                                   threadIdx.x);
 }
 
@@ -211,7 +218,8 @@ static cudaError_t launch_batched_w(const float2* in, float2* out, long long bat
     long long blocks = (batch + per_block - 1) / per_block;
     while (blocks > 0) {  // gridDim.x limit 2^31-1
         long long now = blocks < 0x7fffffffll ? blocks : 0x7fffffffll;
-        kernel<<<(unsigned)now, THREADS, SMEM, stream>>>(in, out, batch, stw, pre, post);
+        const cudaError_t e = launch_dependent(kernel, dim3((unsigned)now), THREADS, SMEM, stream, in, out, batch, stw, pre, post);
+        if (e != cudaSuccess) return e;
         long long done = now * per_block;
         in += done << LOG_L;
         out += done << LOG_L;
@@ -243,8 +251,9 @@ static cudaError_t launch_tiny_t(const float2* in, float2* out, long long batch,
     long long blocks = (batch + PB - 1) / PB;
     while (blocks > 0) {
         long long now = blocks < 0x7fffffffll ? blocks : 0x7fffffffll;
-        if (w) k_tiny<LOG_N, true><<<(unsigned)now, 256, 0, stream>>>(in, out, batch, inverse, pre, post);
-        else k_tiny<LOG_N, false><<<(unsigned)now, 256, 0, stream>>>(in, out, batch, inverse, nullptr, nullptr);
+        const cudaError_t e = launch_dependent(w ? k_tiny<LOG_N, true> : k_tiny<LOG_N, false>, dim3((unsigned)now), 256, 0,
+                                               stream, in, out, batch, inverse, pre, post);
+        if (e != cudaSuccess) return e;
         long long done = now * PB;
         in += done << LOG_N;
         out += done << LOG_N;
@@ -308,7 +317,8 @@ static cudaError_t launch_pass_w(const PassArgs& a, int batch, cudaStream_t stre
     while (batch > 0) {
         int now = batch < 65535 ? batch : 65535;
         grid.y = (unsigned)now;
-        kernel<<<grid, THREADS, SMEM, stream>>>(b);
+        const cudaError_t e = launch_dependent(kernel, grid, THREADS, SMEM, stream, b);
+        if (e != cudaSuccess) return e;
         b.in += (long long)now << a.log2n;
         b.out += (long long)now << a.log2n;
         batch -= now;
@@ -379,8 +389,7 @@ static cudaError_t launch_columns_t(const PassArgs& a, cudaStream_t stream) {
     if (a.log2n > 31 || a.log2n < LOG_L + LOG_C) return cudaErrorInvalidValue;
     PassArgs b = a;
     b.tli = 31;
-    kernel<<<1u << (a.log2n - LOG_L - LOG_C), THREADS, SMEM, stream>>>(b);
-    return cudaGetLastError();
+    return launch_dependent(kernel, dim3(1u << (a.log2n - LOG_L - LOG_C)), THREADS, SMEM, stream, b);
 }
 
 cudaError_t launch_pass_columns(int mode, int log_l, const PassArgs& a, cudaStream_t stream) {

@@ -24,6 +24,28 @@ inline cudaError_t smem_limit(const void* kernel, int bytes, std::atomic<unsigne
     return e;
 }
 
+// Launches a kernel that may start while the stream's previous kernel is still running
+// (programmatic dependent launch): the kernel calls dependent_launch() first and dependent_wait()
+// before it touches the caller's buffers (fft_device.cuh). What a launch, its block scheduling and a
+// kernel's prologue take (1-3 us) then no longer lies between two kernels of a stream. Measured on a
+// B200, calls back to back: one 2^20 transform (two kernels) 16.4 -> 12.7 us, 2^17 10.3 -> 6.1 us,
+// 2^22 41.8 -> 35.1 us, 2^24 139 -> 132 us, 16 x 2^15 12.3 -> 7.1 us, 100003 x 64 20.9 -> 18.5 us.
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
+                                    const A&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Arguments of one pass of the multi-pass decomposition (see k_pass in fft_kernels.cu).
 struct PassArgs {
     const float2* in;

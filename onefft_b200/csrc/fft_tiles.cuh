@@ -97,9 +97,22 @@ __device__ __forceinline__ long long column_dst(const PassArgs& a, unsigned long
     return (long long)(((((k >> a.xlog_blk) << a.xlog_cols) + b) << a.xlog_blk) + (k & ((1ull << a.xlog_blk) - 1)));
 }
 
-// Loads of data the kernel never writes go through the read-only path; the intermediate array
-// between passes may be kept in L2 for the next pass (evict last).
-__device__ __forceinline__ float2 ld_stream(const float2* p) { return __ldg(p); }
+// Loads of the caller's buffers. They are volatile and coherent, not read-only-path loads, so that
+// none moves above the dependent_wait() that orders it after the previous kernel's writes. Data that
+// the kernel itself overwrites (the in-place passes) is loaded through L2 only: blocks of one pass
+// may share a 32-byte sector, and the next kernel, started early on the same SM, could find the copy
+// that a block of this one left in L1 before its neighbour wrote the sector.
+__device__ __forceinline__ float2 ld_stream(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float2 ld_l2(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+// The array between passes may be kept in L2 for the next pass (evict last).
 __device__ __forceinline__ unsigned long long policy_evict_last() {
     unsigned long long pol;
     asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
@@ -222,9 +235,8 @@ __device__ __forceinline__ void batched_tile(const float2* __restrict__ src, flo
 // over the 2^LOG_C L / 16 threads of the tile.
 // W: the first pass multiplies its input by a.pre, the last pass its output by a.post (see
 // PassArgs); without W they are not compiled in.
-// CG: later passes load through L2 only (ld.global.cg), for data that other blocks of the same
-// launch wrote: an SM's L1 may still hold an older copy of a line that it read for a neighbouring
-// transform.
+// CG: later passes load through L2 only (ld_l2), for data that other blocks may have written while
+// this SM's L1 holds an older copy.
 // X: a pass of a column transform (PassArgs' column fields): MODE 0 takes its inter-pass factor
 // from the column fields and, with colstore, writes the column layout (and a.swap_out: it is
 // then the only pass); MODE 2 reads a.in, multiplies by the larger transform's factors and
@@ -263,6 +275,9 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, unsigned t, long lo
         pass_twiddle_rows<LOG_L, LOG_C, MODE>(a, col0, tws, tid, C * T);
         wjf = pass_twiddle_lane<LOG_L>(a, MODE == 0 ? col0 + c : (col0 >> a.log_s) << a.log_s, j);
     }
+    dependent_wait();  // (returns at once in the uneven kernel, whose launches are not dependent ones)
+    const float2 *pre = nullptr, *post = nullptr;
+    if constexpr (W) pre = after_wait(a.pre), post = after_wait(a.post);
     // element j + T k of the column: p0 + k * estep
     const long long estep = (long long)T << a.log_s;
     const long long off0 = toff + base + ((long long)j << a.log_s);
@@ -271,11 +286,10 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, unsigned t, long lo
         const float2* p0 = a.in + off0;
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
-            // The first pass streams the input, which is never read again. Later passes read
-            // and write `out` in place, so they avoid the read-only cache path.
-            float2 x = MODE == 0 ? ld_stream(p0 + k * estep) : CG ? __ldcg(p0 + k * estep) : p0[k * estep];
+            // The first pass streams the input; later passes read and write `out` in place.
+            float2 x = MODE == 0 ? ld_stream(p0 + k * estep) : CG ? ld_l2(p0 + k * estep) : p0[k * estep];
             if constexpr (W && MODE == 0) {
-                if (a.pre) x = cmul(x, __ldg(a.pre + (off0 - toff) + k * estep));
+                if (pre) x = cmul(x, __ldg(pre + (off0 - toff) + k * estep));
             }
             v[k] = a.swap_in ? swap_ri(x) : x;
         }
@@ -332,7 +346,7 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, unsigned t, long lo
         for (int k = 0; k < 16; ++k) {
             float2 x = a.swap_out ? swap_ri(v[k]) : v[k];
             if constexpr (W && MODE == 2) {
-                if (a.post) x = cmul(x, __ldg(a.post + (off0 - toff) + k * estep));
+                if (post) x = cmul(x, __ldg(post + (off0 - toff) + k * estep));
             }
             if (MODE == 1 && a.l2_keep) st_policy(p0 + k * estep, x, keep);
             else p0[k * estep] = x;

@@ -192,6 +192,7 @@ __device__ __forceinline__ bool tma_tile(const PassArgs& a, const CUtensorMap* t
         else asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         go = ready();
         if (go) {
+            dependent_wait();  // the other threads touch the caller's buffers only after the copy landed
             mbar_expect_tx(bar, (unsigned)(C * L * sizeof(float2)));
             // With l2_keep the array between passes should stay in L2: the input (read once)
             // and the last pass's tile (read for the last time) are loaded evict-first.
@@ -231,6 +232,11 @@ __device__ __forceinline__ bool tma_tile(const PassArgs& a, const CUtensorMap* t
         }
         return false;
     }
+    const float2 *pre = nullptr, *post = nullptr;
+    if constexpr (W) {
+        dependent_wait();  // this thread reads the caller's weights itself
+        pre = after_wait(a.pre), post = after_wait(a.post);
+    }
     landed();
     float2 v[16];
 #pragma unroll
@@ -238,7 +244,7 @@ __device__ __forceinline__ bool tma_tile(const PassArgs& a, const CUtensorMap* t
         float2 x = smem[(j + T * k) * C + c];
         // input element col0 + c + (j + T k) S of the transform (first pass only)
         if constexpr (W && MODE == 0) {
-            if (a.pre) x = cmul(x, __ldg(a.pre + col0 + c + ((unsigned)(j + T * k) << a.log_s)));
+            if (pre) x = cmul(x, __ldg(pre + col0 + c + ((unsigned)(j + T * k) << a.log_s)));
         }
         v[k] = a.swap_in ? swap_ri(x) : x;
     }
@@ -294,8 +300,8 @@ __device__ __forceinline__ bool tma_tile(const PassArgs& a, const CUtensorMap* t
             float2 x = a.swap_out ? swap_ri(v[k]) : v[k];
             // output element q0 + c + (j + T k) S + h L S of the transform, natural order (last pass)
             if constexpr (W && MODE == 2) {
-                if (a.post)
-                    x = cmul(x, __ldg(a.post + (unsigned)(q0 + c) + ((unsigned)(j + T * k) << a.log_s) +
+                if (post)
+                    x = cmul(x, __ldg(post + (unsigned)(q0 + c) + ((unsigned)(j + T * k) << a.log_s) +
                                      ((unsigned)h << (a.log_s + LOG_L))));
             }
             smem[(j + T * k) * C + c] = x;
@@ -316,6 +322,7 @@ __global__ void __launch_bounds__(1 << (LOG_L + LOG_C - 4), (X ? 0 : tma_min_blo
     k_pass_tma(PassArgs a, const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout) {
     extern __shared__ __align__(1024) float2 smem[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + tma_bar_offset(LOG_L, LOG_C));
+    dependent_launch();
     if (smem_u32(smem) & 127) {  // bulk tensor copies need a 128-byte aligned destination
         if (threadIdx.x == 0) *(volatile unsigned*)a.err = 2u;
         return;
@@ -602,8 +609,7 @@ static cudaError_t launch_tma_w(const PassArgs& a, int batch, cudaStream_t strea
     dim3 grid(a.ntiles ? a.ntiles : 1u << (a.log2n - LOG_L - LOG_C), (unsigned)batch, 1);
     PassArgs b = a;
     if (!a.ntiles) b.tli = 31;
-    kernel<<<grid, THREADS, SMEM, stream>>>(b, tin, tout);
-    return cudaGetLastError();
+    return launch_dependent(kernel, grid, THREADS, SMEM, stream, b, tin, tout);
 }
 
 // Tile shapes with a TMA kernel (the only ones pass_tma_supported accepts): widths 2 .. 16
@@ -695,8 +701,7 @@ static cudaError_t launch_columns_tma_t(const PassArgs& a, cudaStream_t stream) 
     if (!make_map(&tin, a.in, MODE, a.log2n, LOG_L, LOG_C, a.log_s, 1)) return cudaErrorInvalidValue;
     PassArgs b = a;
     b.tli = 31;
-    kernel<<<1u << (a.log2n - LOG_L - LOG_C), THREADS, SMEM, stream>>>(b, tin, tin);
-    return cudaGetLastError();
+    return launch_dependent(kernel, dim3(1u << (a.log2n - LOG_L - LOG_C)), THREADS, SMEM, stream, b, tin, tin);
 }
 
 cudaError_t launch_pass_columns_tma(int mode, int log_l, const PassArgs& a, cudaStream_t stream) {

@@ -1,0 +1,46 @@
+"""GPU test of the dependent launches: a kernel may start while its predecessor in the stream still
+runs, so a chain of calls that each read what the one before wrote (in two buffers in turn, the weights
+of the next call included) and that nothing waits between must give the bits of the same chain with a
+synchronisation after every call. Sizes: both sides of the 1184-block line of the early release, one,
+two and three kernels a call, tiny and batched kernels, TMA and plain passes (8-byte aligned buffers).
+"""
+from __future__ import annotations
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("log2n,batch", [(3, 1), (3, 700001), (6, 100003), (9, 37), (10, 1), (12, 1183), (12, 1185),
+                                         (14, 3), (15, 1), (16, 9), (17, 5), (18, 3), (20, 1), (20, 5), (22, 1), (24, 1)])
+@pytest.mark.parametrize("shift", [0, 1])  # offset of every buffer in complex values: 1 = not 16-byte aligned
+def test_unsynchronised_chain_same_bits(ofb, log2n, batch, shift):
+    import torch
+    n = 1 << log2n
+    values = n * batch
+    g = torch.Generator(device="cuda").manual_seed(1000 * log2n + batch)
+    x = torch.randn(2 * (values + 1), device="cuda", generator=g) / n ** 0.5
+    plan = ofb.Plan(n)
+    stream = torch.cuda.current_stream().cuda_stream
+    out = []
+    for sync in (True, False):
+        a, b = x.clone(), torch.zeros_like(x)
+        pa, pb = a.data_ptr() + 8 * shift, b.data_ptr() + 8 * shift
+        if not sync:
+            torch.cuda.synchronize()
+        for i in range(6):
+            for call in (lambda: plan.dev_forward(pa, pb, batch, stream),
+                         lambda: plan.dev_inverse(pb, pa, batch, stream),
+                         # one transform, windowed by what the call before wrote last
+                         lambda: plan.dev_weighted(pb, pb + 8 * n, 1, pa + 8 * (values - n), None, False, stream)
+                         if batch > 2 else None):
+                call()
+                if sync:
+                    torch.cuda.synchronize()
+            if log2n > 0:  # keep the magnitudes: the pair multiplies by n
+                a.mul_(1.0 / n)
+        torch.cuda.synchronize()
+        plan.check()
+        out.append((a, b))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    assert bool(torch.isfinite(out[0][0]).all())
