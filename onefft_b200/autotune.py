@@ -193,7 +193,8 @@ PIPELINED = 15
 def batched_log_c_candidates(l: int) -> list[int]:
     """Transforms per block (log2) compiled for the one-kernel size 2^l (fft_kernels.cu,
     batched_log_c_supported): the default 4096 / n, half and twice that up to 8192 values; at 2^12
-    and 2^13 also the pipelined form (fft_tma.cu, batched_pipe_supported)."""
+    also the pipelined form (fft_tma.cu, batched_pipe_supported); 2^13 and 2^14 run pipelined
+    whatever the width (fft_long.cu)."""
     b = max(0, 12 - l)
     out = [c for c in (b - 1, b, b + 1) if c == b or (c >= 0 and l + c <= 13)]
     return out + ([PIPELINED] if l in (12, 13) else [])

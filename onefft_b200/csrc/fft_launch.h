@@ -121,19 +121,25 @@ bool pass_tma_supported(int log_l, int log_c);
 // Test hook: every first bounded wait of the TMA-staged kernels on the current device counts as
 // expired while `on` (onefft_debug_expire_waits).
 cudaError_t set_expire_waits(int on);
+cudaError_t set_expire_waits_long(int on);  // fft_long.cu's part of it
 // Passes 0 and 1 of a three-pass transform (pass lengths 2^l0, 2^l1, 2^len2, tile widths 2^c0,
 // 2^c1) in ONE persistent launch over chunks of 2^g last-digit columns, pass 1 trailing pass 0 by
 // `lag` chunks (fft_tma.cu, k_pass01_fused). a0 / a1: the arguments of the chunked launches of
 // passes 0 and 1 (ntiles = tiles per chunk; the per-chunk bases are ignored); one transform.
 // ctr: 2 + 2^(len2 - g) zeroed words used by no concurrent launch (zero again afterwards).
 bool pass01_fused_supported(int l0, int c0, int l1, int c1);
-// One-kernel sizes 2^12 / 2^13 as a persistent kernel with one transform per block and the next
+// One-kernel size 2^12 as a persistent kernel with one transform per block and the next
 // transform's values arriving by one bulk copy while the current one computes (fft_tma.cu,
 // k_batched_pipe); same bits as launch_single_kernel. `in` 16-byte aligned; err: the plan's error
 // word (an expired copy wait).
 bool batched_pipe_supported(int log2n);
 cudaError_t launch_batched_pipe(int log2n, const float2* in, float2* out, long long batch, const float2* stw,
                                 int inverse, unsigned* err, cudaStream_t stream);
+// 2^13 and 2^14 as persistent blocks with the next transform's copy in flight (fft_long.cu,
+// k_batched_long); same bits as launch_single_kernel. `in` 16-byte aligned, err as above.
+bool batched_long_supported(int log2n);
+cudaError_t launch_batched_long(int log2n, const float2* in, float2* out, long long batch, const float2* stw,
+                                int inverse, unsigned* err, cudaStream_t stream, const float2* pre, const float2* post);
 cudaError_t launch_pass01_fused(int l0, int c0, int l1, int c1, const PassArgs& a0, const PassArgs& a1, int g,
                                 int len2, int lag, unsigned* ctr, cudaStream_t stream);
 cudaError_t launch_pass_tma(int mode, int log_l, int log_c, const PassArgs& a, int batch, cudaStream_t stream);

@@ -181,14 +181,14 @@ static Shape tuned_shape(int m) {
 }
 
 // One kernel, cols[0] = this: the persistent pipelined kernel (launch_batched_pipe) instead of
-// k_batched (ONEFFT_COLS_PIPELINED in onefft_cuda.h).
+// k_batched at 2^12 (ONEFFT_COLS_PIPELINED in onefft_cuda.h; 2^13 is pipelined whatever the width).
 constexpr int kPipelinedCols = 15;
 
 static bool valid_shape(int m, const Shape &s) {
     if (s.npass == 1)
         return s.len[0] == m && m <= kMaxSingleLog2 &&
                (s.cols[0] == -1 || batched_log_c_supported(m, s.cols[0]) ||
-                (s.cols[0] == kPipelinedCols && batched_pipe_supported(m)));
+                (s.cols[0] == kPipelinedCols && (batched_pipe_supported(m) || m == 13)));
     if (s.npass < 2 || s.npass > 3) return false;
     int sum = 0;
     for (int p = 0; p < s.npass; ++p) {
@@ -444,6 +444,10 @@ static cudaError_t plan_enqueue(const onefft_plan *p, const float2 *in, float2 *
     if (p->npass == 1) {
         g_launches.fetch_add(1);
         if (p->tc) return launch_single_kernel_tc(p->log2n, in, out, batch, p->stw[0], inverse, p->tc, s);
+        // 2^13 and 2^14 through bulk copies where the input allows them (k_batched otherwise: 5-20 %
+        // slower from 150 transforms on, a tick slower below; the same bits)
+        if (batched_long_supported(p->log2n) && !((uintptr_t)in & 15))
+            return launch_batched_long(p->log2n, in, out, batch, p->stw[0], inverse, p->err, s, pre, post);
         if (p->cols[0] == kPipelinedCols) {
             // bulk copies need 16-byte aligned transforms; weighted calls use k_batched's weights
             if (!pre && !post && !((uintptr_t)in & 15))
