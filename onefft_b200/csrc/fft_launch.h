@@ -122,6 +122,7 @@ bool pass_tma_supported(int log_l, int log_c);
 // expired while `on` (onefft_debug_expire_waits).
 cudaError_t set_expire_waits(int on);
 cudaError_t set_expire_waits_long(int on);  // fft_long.cu's part of it
+cudaError_t set_expire_waits_wide(int on);  // fft_wide.cu's
 // Passes 0 and 1 of a three-pass transform (pass lengths 2^l0, 2^l1, 2^len2, tile widths 2^c0,
 // 2^c1) in ONE persistent launch over chunks of 2^g last-digit columns, pass 1 trailing pass 0 by
 // `lag` chunks (fft_tma.cu, k_pass01_fused). a0 / a1: the arguments of the chunked launches of
@@ -143,6 +144,9 @@ cudaError_t launch_batched_long(int log2n, const float2* in, float2* out, long l
 cudaError_t launch_pass01_fused(int l0, int c0, int l1, int c1, const PassArgs& a0, const PassArgs& a1, int g,
                                 int len2, int lag, unsigned* ctr, cudaStream_t stream);
 cudaError_t launch_pass_tma(int mode, int log_l, int log_c, const PassArgs& a, int batch, cudaStream_t stream);
+// Wide-tile persistent passes (fft_wide.cu): same arithmetic, arguments and requirements as
+// launch_pass_tma (no chunks); the shapes the tuned table marks (onefft_api.cu, kWideTile)
+cudaError_t launch_pass_wide(int mode, int log_l, int log_c, const PassArgs& a, int batch, cudaStream_t stream);
 // split-BF16 tensor-core variants (fft_tc.cu) of `terms` = 3 or 6 split products: n = 2^4 .. 2^14
 // in one kernel; pass lengths 2^5 .. 2^12 with the default tile width pass_log_c()
 cudaError_t launch_single_kernel_tc(int log2n, const float2* in, float2* out, long long batch, const float2* stw,

@@ -18,8 +18,9 @@ namespace ofb {
 
 cudaError_t set_expire_waits(int on) {
     const int v = on ? 1 : 0;
-    const cudaError_t e = cudaMemcpyToSymbol(g_expire_waits, &v, sizeof v);
-    return e == cudaSuccess ? set_expire_waits_long(v) : e;
+    cudaError_t e = cudaMemcpyToSymbol(g_expire_waits, &v, sizeof v);
+    if (e == cudaSuccess) e = set_expire_waits_long(v);
+    return e == cudaSuccess ? set_expire_waits_wide(v) : e;
 }
 
 // Blocks per SM that the register allocation must allow (0: the compiler chooses freely). Measured

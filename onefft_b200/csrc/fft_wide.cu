@@ -1,0 +1,303 @@
+// Wide-tile pass kernels (sm_100a): one pass of a two- or three-pass transform by persistent blocks,
+// one tile of 2^14 (or two of 2^13) values per SM, with the next tile's bulk tensor copy in flight
+// while the current one computes. Same arithmetic as k_pass and k_pass_tma on the same values.
+//
+// Why beside k_pass_tma (one tile per block, 16 values per thread): its tiles of 2^11 .. 2^12
+// values need many blocks per SM to hide their copies, which registers allow only for short columns:
+// at 2048 or 4096 values a column, one or two blocks ran and waited. So 2^22 .. 2^24 took three
+// passes of short columns over HBM; here two passes of long ones are faster. A thread owns one
+// butterfly lane of TWO adjacent columns, 32 values: it loads each stage twiddle once for both,
+// moves 16-byte pieces from the landing buffer and to strided outputs, and 8-byte words (two columns'
+// re parts, then their im parts) through the exchange buffer, which with half the bytes per round
+// leaves the room for the landing buffer. The first pass regroups its threads in the last exchange,
+// so that it stores contiguous runs straight from registers (k_pass_tma transposes once more).
+//
+// What bounds it (B200, a pass over 2^24 values, 268 MB moved, 41 us at the copy rate): the tile's
+// load, arithmetic and store between the block's barriers. First pass, columns x values: 2 x 4096
+// 65 us, 4 x 2048 59, 8 x 1024 56, 16 x 512 52, 32 x 256 50; last pass 4 x 4096 69 (without its
+// 32-byte store pieces 61), 8 x 2048 62, 16 x 1024 60, 16 x 512 50. Loads and stores alone, no
+// arithmetic: 58, 50, 48, 48, 46; 55, 52, 50, 45. Sustained, the HBM traffic of a plain copy alone draws
+// the board's 1000 W, so arithmetic beside it lowers the clock: fewer passes pay twice.
+//
+// Measured and left out: inter-pass powers shared by the block (the extra latency costs what the
+// FP64 work saves), stage twiddles loaded before the exchange that precedes their stage (no
+// change), strided last passes of 8 columns at strides of 512 KiB and more (64-byte pieces:
+// 2^27 1478 us against 1228 with 16 columns).
+#include "fft_tma.cuh"
+
+namespace ofb {
+
+cudaError_t set_expire_waits_wide(int on) {
+    const int v = on ? 1 : 0;
+    return cudaMemcpyToSymbol(g_expire_waits, &v, sizeof v);
+}
+
+// Geometry of a tile of C = 2^LOG_C columns of L = 2^LOG_L values. A thread owns one of the T = L / 16
+// butterfly lanes of TWO adjacent columns: it loads each stage twiddle once for both, and moves the
+// two columns' re (then im) parts through the exchange buffer as one 8-byte word.
+template <int LOG_L, int LOG_C>
+struct Wide {
+    static constexpr int L = 1 << LOG_L, C = 1 << LOG_C, P = C / 2, T = L / 16, THREADS = T * P;
+    static constexpr int VALUES = L * C;
+    // Exchange buffer, in 8-byte words: rows [e][p] of the column pairs with one pad row every 16, or
+    // whole columns [p][e] for the exchange that regroups the threads by column (padded alike, and
+    // offset so that the writers, 16 / P lanes of each pair, meet distinct banks).
+    static constexpr int COL = L + L / 16 + 16 / P;
+    static_assert(P <= 16 && (L / 16) % 16 == 0, "bank layout");
+    static constexpr int ROW_WORDS = (L + L / 16) * P, COL_WORDS = COL * P;
+    static constexpr int EX_WORDS = ROW_WORDS > COL_WORDS ? ROW_WORDS : COL_WORDS;
+    static constexpr int EX_OFF = 8 * VALUES;                     // bytes; the landing buffer comes first
+    static constexpr int TW_OFF = EX_OFF + 8 * EX_WORDS;          // 2 x C x 17 inter-pass factors
+    static constexpr int BAR_OFF = TW_OFF + 2 * C * 17 * 8;
+    static constexpr int SMEM = BAR_OFF + 16;
+};
+
+// Stage S on lane j of both columns (stage_compute, with each twiddle loaded once).
+template <int LOG_L, int S>
+__device__ __forceinline__ void pair_stage(float2 (&v)[2][16], int j, const float2* __restrict__ stw) {
+    using St = Stages<LOG_L>;
+    constexpr int LR = St::log2_radix(S), R = 1 << LR, NS = 1 << St::log2_ns(S), BPT = 16 / R;
+#pragma unroll
+    for (int i = 0; i < BPT; ++i) {
+        float2 a[2][R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) a[0][q] = v[0][i + BPT * q], a[1][q] = v[1][i + BPT * q];
+        if (S > 0) {
+            const float2* tw = stw + St::tw_offset(S) + ((j + St::T * i) & (NS - 1));
+#pragma unroll
+            for (int q = 1; q < R; ++q) {
+                const float2 w = __ldg(tw + (q - 1) * NS);
+                a[0][q] = cmul(a[0][q], w);
+                a[1][q] = cmul(a[1][q], w);
+            }
+        }
+        dft<R>(a[0]);
+        dft<R>(a[1]);
+#pragma unroll
+        for (int p = 0; p < R; ++p) v[0][i + BPT * p] = a[0][p], v[1][i + BPT * p] = a[1][p];
+    }
+}
+
+// The exchange between stages S and S + 1 (tile_fft's): output p of lane j goes to element
+// E0(j) + p Ns of pair c, and element jr + T k of pair cr is read back, re and im parts one after
+// the other. COLUMNS: the buffer holds whole columns, so that the readers can run along a column
+// where the writers ran across columns. The block has been synchronised since the buffer was last
+// read.
+template <int LOG_L, int LOG_C, int S, bool COLUMNS>
+__device__ __forceinline__ void pair_exchange(float2 (&v)[2][16], int j, int c, int jr, int cr, float2* ex) {
+    using G = Wide<LOG_L, LOG_C>;
+    constexpr int LNS = Stages<LOG_L>::log2_ns(S), NS = 1 << LNS;
+    constexpr int STEP = COLUMNS ? 1 : G::P;
+    const int e0 = ((j >> LNS) << (4 + LNS)) + (j & (NS - 1));
+    float2* w = ex + (COLUMNS ? c * G::COL + spad(e0) : spad(e0) * STEP + c);
+    const float2* r = ex + (COLUMNS ? cr * G::COL + spad(jr) : spad(jr) * STEP + cr);
+#pragma unroll
+    for (int p = 0; p < 16; ++p) w[padc(p * NS) * STEP] = make_float2(v[0][p].x, v[1][p].x);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const float2 x = r[padc(k * G::T) * STEP];
+        v[0][k].x = x.x, v[1][k].x = x.y;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < 16; ++p) w[padc(p * NS) * STEP] = make_float2(v[0][p].y, v[1][p].y);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const float2 x = r[padc(k * G::T) * STEP];
+        v[0][k].y = x.x, v[1][k].y = x.y;
+    }
+}
+
+// Stages S .. of the tile; the last one runs on lane jl of pair cl.
+template <int LOG_L, int LOG_C, int S, bool REGROUP>
+__device__ __forceinline__ void pair_stages(float2 (&v)[2][16], int j, int c, int jl, int cl,
+                                            const float2* __restrict__ stw, float2* ex) {
+    constexpr int COUNT = Stages<LOG_L>::COUNT;
+    pair_stage<LOG_L, S>(v, S + 1 == COUNT ? jl : j, stw);
+    if constexpr (S + 1 < COUNT) {
+        constexpr bool TO_LAST = S + 2 == COUNT;
+        if constexpr (S > 0) __syncthreads();  // the previous exchange's reads are done
+        pair_exchange<LOG_L, LOG_C, S, TO_LAST && REGROUP>(v, j, c, TO_LAST ? jl : j, TO_LAST ? cl : c, ex);
+        pair_stages<LOG_L, LOG_C, S + 1, REGROUP>(v, j, c, jl, cl, stw, ex);
+    }
+}
+
+template <int LOG_L, int LOG_C, int MODE, bool SWAP, bool W>
+__global__ void __launch_bounds__(Wide<LOG_L, LOG_C>::THREADS, LOG_L + LOG_C >= 14 ? 1 : LOG_L + LOG_C == 13 ? 2 : 4)
+    k_pass_wide(PassArgs a, const __grid_constant__ CUtensorMap tin, unsigned tiles, int log_tiles) {
+    using G = Wide<LOG_L, LOG_C>;
+    extern __shared__ __align__(1024) unsigned char wide_smem[];
+    const float2* land = reinterpret_cast<const float2*>(wide_smem);
+    float2* ex = reinterpret_cast<float2*>(wide_smem + G::EX_OFF);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(wide_smem + G::BAR_OFF);
+    const int tid = threadIdx.x;
+    dependent_launch();
+    if (smem_u32(wide_smem) & 127) {  // bulk tensor copies need a 128-byte aligned destination
+        if (tid == 0) *(volatile unsigned*)a.err = 2u;
+        return;
+    }
+    // loads, first stages and strided stores run across the columns, contiguous stores along them
+    const int c = tid & (G::P - 1), j = tid / G::P;
+    const int cl = MODE == 0 ? tid / G::T : c, jl = MODE == 0 ? tid & (G::T - 1) : j;
+    auto load = [&](unsigned t) {
+        const int b = (int)(t >> log_tiles);
+        const unsigned col0 = (t & ((1u << log_tiles) - 1)) << LOG_C;
+        mbar_expect_tx(bar, (unsigned)(G::VALUES * sizeof(float2)));
+        if (MODE == 0) tma_load_4d(wide_smem, &tin, (int)col0, 0, 0, b, bar);
+        else tma_load_5d(wide_smem, &tin, (int)(col0 & ((1u << a.log_s) - 1)), 0, 0, (int)(col0 >> a.log_s), b, bar);
+    };
+    unsigned t = blockIdx.x, parity = 0;
+    if (t >= tiles) return;
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        dependent_wait();  // the other threads touch the caller's buffers only after the copy landed
+        load(t);
+    }
+    const float2 *pre = nullptr, *post = nullptr;
+    if constexpr (W) {
+        dependent_wait();  // every thread reads the caller's weights
+        pre = after_wait(a.pre), post = after_wait(a.post);
+    }
+    __syncthreads();  // the barrier is initialised before anyone waits on it
+    for (; t < tiles; t += gridDim.x, parity ^= 1u) {
+        const unsigned col0 = (t & ((1u << log_tiles) - 1)) << LOG_C;
+        const long long toff = (long long)(t >> log_tiles) << a.log2n;
+        // inter-pass factors (as pass_tile) while the copy is in flight; the rows alternate between
+        // two buffers, since slower threads may still read the previous tile's
+        float2* tws = reinterpret_cast<float2*>(wide_smem + G::TW_OFF) + parity * (G::C * 17);
+        float2 wl[2];
+        if (MODE != 2) {
+            pass_twiddle_rows<LOG_L, LOG_C, MODE>(a, col0, tws, tid, G::THREADS);
+            const unsigned f = MODE == 0 ? col0 + 2 * cl : (col0 >> a.log_s) << a.log_s;
+            wl[0] = pass_twiddle_lane<LOG_L>(a, f, jl);
+            wl[1] = MODE == 0 ? pass_twiddle_lane<LOG_L>(a, f + 1, jl) : wl[0];
+        }
+        const bool ok = !g_expire_waits && mbar_wait(bar, parity);
+        float2 v[2][16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const float4 x = *reinterpret_cast<const float4*>(land + (j + G::T * k) * G::C + 2 * c);
+            v[0][k] = make_float2(x.x, x.y);
+            v[1][k] = make_float2(x.z, x.w);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                if constexpr (W && MODE == 0) {
+                    if (pre) v[i][k] = cmul(v[i][k], __ldg(pre + col0 + 2 * c + i + ((unsigned)(j + G::T * k) << a.log_s)));
+                }
+                if (SWAP && MODE == 0) v[i][k] = swap_ri(v[i][k]);
+            }
+        }
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0) {
+                *(volatile unsigned*)a.err = 1u;
+                mbar_wait(bar, parity);  // let a late copy land before the memory is released
+            }
+            return;
+        }
+        // every value is in registers: the landing buffer takes the next tile
+        if (tid == 0 && t + gridDim.x < tiles) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            load(t + gridDim.x);
+        }
+        pair_stages<LOG_L, LOG_C, 0, MODE == 0>(v, j, c, jl, cl, a.stw, ex);
+        if (MODE != 2) {
+            const float2* tw = tws + (MODE == 0 ? 2 * cl * 17 : 0);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                v[0][k] = cmul(v[0][k], cmul(wl[0], tw[k]));
+                v[1][k] = cmul(v[1][k], cmul(wl[1], tw[MODE == 0 ? 17 + k : k]));
+            }
+        }
+        if (MODE == 0) {
+            // contiguous column runs at their digit-reversed place, as k_pass
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const unsigned rr = col0 + 2 * cl + i, j2 = rr & ((1u << a.rev_b2) - 1), j1 = rr >> a.rev_b2;
+                float2* q = a.out + toff + (((j1 + (j2 << a.rev_b1)) << LOG_L) + jl);
+#pragma unroll
+                for (int k = 0; k < 16; ++k) q[G::T * k] = v[i][k];
+            }
+        } else {
+            const unsigned q0 = col0 & ((1u << a.log_s) - 1), h = col0 >> a.log_s;
+            const unsigned base = q0 + 2 * c + (h << (a.log_s + LOG_L));
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                const unsigned e = base + ((unsigned)(j + G::T * k) << a.log_s);
+                float2 y[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    y[i] = SWAP && MODE == 2 ? swap_ri(v[i][k]) : v[i][k];
+                    if constexpr (W && MODE == 2) {
+                        if (post) y[i] = cmul(y[i], __ldg(post + e + i));
+                    }
+                }
+                *reinterpret_cast<float4*>(a.out + toff + e) = make_float4(y[0].x, y[0].y, y[1].x, y[1].y);
+            }
+        }
+    }
+}
+
+template <int LOG_L, int LOG_C, int MODE, bool SWAP, bool W>
+static cudaError_t launch_wide_w(const PassArgs& a, int batch, cudaStream_t stream) {
+    using G = Wide<LOG_L, LOG_C>;
+    auto kernel = k_pass_wide<LOG_L, LOG_C, MODE, SWAP, W>;
+    static std::atomic<unsigned long long> done{0};
+    cudaError_t e = smem_limit((const void*)kernel, G::SMEM, done);
+    if (e != cudaSuccess) return e;
+    // persistent grid: the blocks that fit on the device at once (per device, computed once)
+    static std::atomic<int> grid_of[64];
+    int dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    int grid = grid_of[dev & 63].load(std::memory_order_relaxed);
+    if (grid == 0) {
+        int per_sm = 0, sms = 0;
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, G::THREADS, G::SMEM)) != cudaSuccess) return e;
+        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+        grid = per_sm * sms > 0 ? per_sm * sms : 1;
+        grid_of[dev & 63].store(grid, std::memory_order_relaxed);
+    }
+    CUtensorMap tin;
+    if (!make_map(&tin, MODE == 0 ? a.in : a.out, MODE, a.log2n, LOG_L, LOG_C, a.log_s, batch))
+        return cudaErrorInvalidValue;
+    const int log_tiles = a.log2n - LOG_L - LOG_C;
+    const unsigned tiles = (unsigned)batch << log_tiles;
+    if ((unsigned)grid > tiles) grid = (int)tiles;
+    return launch_dependent(kernel, dim3((unsigned)grid), G::THREADS, G::SMEM, stream, a, tin, tiles, log_tiles);
+}
+
+template <int LOG_L, int LOG_C, int MODE>
+static cudaError_t launch_wide_t(const PassArgs& a, int batch, cudaStream_t stream) {
+    const bool swap = MODE == 0 ? a.swap_in : a.swap_out;
+    if constexpr (MODE != 1) {
+        if (MODE == 0 ? a.pre != nullptr : a.post != nullptr)
+            return swap ? launch_wide_w<LOG_L, LOG_C, MODE, true, true>(a, batch, stream)
+                        : launch_wide_w<LOG_L, LOG_C, MODE, false, true>(a, batch, stream);
+        if (swap) return launch_wide_w<LOG_L, LOG_C, MODE, true, false>(a, batch, stream);
+    }
+    return launch_wide_w<LOG_L, LOG_C, MODE, false, false>(a, batch, stream);
+}
+
+// Tile shapes (log2 values, log2 columns) with a wide kernel, by pass: those the tuned table uses.
+#define OFB_WIDE_FIRST(X) X(12, 1) X(11, 2) X(10, 4) X(10, 3) X(9, 4) X(8, 5)
+#define OFB_WIDE_MIDDLE(X) X(10, 4) X(9, 4) X(8, 5)
+#define OFB_WIDE_LAST(X) X(12, 2) X(11, 3) X(10, 4) X(10, 3) X(9, 4) X(8, 4)
+
+cudaError_t launch_pass_wide(int mode, int log_l, int log_c, const PassArgs& a, int batch, cudaStream_t stream) {
+#define OFB_WIDE_CASE0(LL, LC) \
+    if (mode == 0 && log_l == LL && log_c == LC) return launch_wide_t<LL, LC, 0>(a, batch, stream);
+#define OFB_WIDE_CASE1(LL, LC) \
+    if (mode == 1 && log_l == LL && log_c == LC) return launch_wide_t<LL, LC, 1>(a, batch, stream);
+#define OFB_WIDE_CASE2(LL, LC) \
+    if (mode == 2 && log_l == LL && log_c == LC) return launch_wide_t<LL, LC, 2>(a, batch, stream);
+    OFB_WIDE_FIRST(OFB_WIDE_CASE0)
+    OFB_WIDE_MIDDLE(OFB_WIDE_CASE1)
+    OFB_WIDE_LAST(OFB_WIDE_CASE2)
+#undef OFB_WIDE_CASE0
+#undef OFB_WIDE_CASE1
+#undef OFB_WIDE_CASE2
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace ofb

@@ -116,10 +116,19 @@ struct onefft_plan {
     void *mem;             // the one device allocation
     size_t mem_bytes;
     const float2 *stw[3];  // stage twiddles of each pass's length
+    // The passes of calls whose buffers do not allow bulk tensor copies, where the tuned table has
+    // others for them (plain_npass > 0): lengths, tile widths, stage twiddles
+    int plain_npass, plain_len[3], plain_cols[3];
+    const float2 *plain_stw[3];
+    int plain_l2_keep;
     const double2 *tw_lo;  // two-level FP64 tables of w_n (npass >= 2)
     const double2 *tw_hi;
     int lo_bits;
 };
+
+// Tile width flag of the tuned table: the pass runs through its wide-tile kernel (launch_pass_wide)
+// where the buffers allow bulk tensor copies.
+constexpr int kWideTile = 16;
 
 // How a size runs: number of passes, their lengths and tile widths. The table below is the
 // tuned choice per log2 n (onefft_b200/autotune.py measures the candidates on the device and
@@ -134,33 +143,67 @@ struct Shape {
     int fuse_lag = 0;  // the tuned table leaves it out: no size runs the fused passes by default
 };
 
-// Fastest shapes measured on a B200 by onefft_b200/autotune.py (forward transform, L2 flushed
-// before each repetition): {npass, {log2 lengths}, {log2 tile widths}, l2_keep, chunk, tma}.
-// 2^16 keeps the (8, 8) split (as fast as the best) so the uneven batch's in-block passes,
-// which use it, stay bit-identical to this path.
+// Shapes by size: {npass, {log2 lengths}, {log2 tile widths}, l2_keep, chunk, tma}; W(c): the wide-tile
+// kernel with 2^c columns (fft_wide.cu), else k_pass_tma (tma) or k_pass. Timed on a B200 with calls
+// back to back on three buffer pairs in turn, warm for 0.3 s (the clock then sits where the board's
+// power limit leaves it), single transforms and batches up to 2^26 values; one shape per size,
+// so that a transform's bits do not depend on its batch. us, this table against the shapes before it
+// (all with dependent launches), at batch 1 / a small batch / a large one:
+//   2^17 (10,7)     5.6 / 36.0 (32) / 262 (256)  ->  6.7 / 27.4 / 199
+//   2^18 (10,8)     6.6 / 33.8 (16) / 248 (128)  ->  8.0 / 28.8 / 204
+//   2^19 (8,11)     9.0 / 43.5 (8)  / 315 (64)   ->  9.2 / 29.0 / 212
+//   2^20 (12,8)    13.2 / 28.4 (3)  / 258 (32)   -> 11.0 / 26.3 / 217
+//   2^21 (11,10)   21.7 / 53.0 (3)  / 272 (16)   -> 19.9 / 47.6 / 223
+//   2^22 (8,7,7)   35.4 / 99.9 (3)  / 281 (8)    -> 36.3 / 95.9 / 231
+//   2^23 (8,8,7)   62.6 /             288 (4)    -> 67.5 /        240
+//   2^24 (8,8,8)   143  /             281 (2)    -> 132  /        254
+//   2^26 (8,8,10)  586 -> 575;  2^27 (8,9,10) 1228 -> 1155;  2^28 (10,10,8) 2702 -> (9,9,10) 2408;
+//   2^29 (10,10,9) 5534 -> (9,10,10) 5162;  2^30 (10,11,9) 11499 -> (10,10,10) 10571
+// 2^15, 2^16 and 2^25 keep k_pass_tma: no wide shape was faster (2^16 in (8,8), also the split of the
+// uneven batch's in-block passes, which stay bit-identical to this path).
+constexpr int W(int c) { return kWideTile | c; }
 static const Shape kTuned[] = {
     /* 15 */ {2, {8, 7, 0}, {3, 4, 0}, 0, 0, 1},
     /* 16 */ {2, {8, 8, 0}, {3, 3, 0}, 0, 0, 1},
+    /* 17 */ {2, {8, 9, 0}, {3, 3, 0}, 0, 0, 1},
+    /* 18 */ {2, {10, 8, 0}, {W(3), 3, 0}, 0, 0, 1},
+    /* 19 */ {2, {11, 8, 0}, {W(2), W(4), 0}, 0, 0, 1},
+    /* 20 */ {2, {10, 10, 0}, {W(3), W(3), 0}, 0, 0, 1},
+    /* 21 */ {2, {11, 10, 0}, {W(2), W(3), 0}, 0, 0, 1},
+    /* 22 */ {2, {11, 11, 0}, {W(2), W(3), 0}, 0, 0, 1},
+    /* 23 */ {2, {12, 11, 0}, {W(1), W(3), 0}, 0, 0, 1},
+    /* 24 */ {2, {12, 12, 0}, {W(1), W(2), 0}, 0, 0, 1},
+    /* 25 */ {3, {8, 8, 9}, {3, 3, 3}, 0, 0, 1},
+    /* 26 */ {3, {9, 8, 9}, {W(4), W(5), W(4)}, 0, 0, 1},
+    /* 27 */ {3, {8, 9, 10}, {W(5), W(4), W(4)}, 0, 0, 1},
+    /* 28 */ {3, {9, 9, 10}, {W(4), W(4), W(4)}, 0, 0, 1},
+    /* 29 */ {3, {9, 10, 10}, {W(4), W(4), W(4)}, 0, 0, 1},
+    /* 30 */ {3, {10, 10, 10}, {W(4), W(4), W(4)}, 0, 0, 1},
+};
+static_assert(sizeof(kTuned) / sizeof(kTuned[0]) == 30 - 15 + 1, "one shape per size 2^15 .. 2^30");
+
+// The passes of calls whose buffers do not allow bulk tensor copies (not 16-byte aligned, or more
+// than 65535 transforms), 2^17 .. 2^30: per-thread loads run the long columns of the shapes above in
+// blocks of 1024 threads, one per SM (2^24 in (12,12) 217 us against 185 in (8,8,8), 2^23 107
+// against 91, 2^28 3574 against 3438).
+static const Shape kPlain[] = {
     /* 17 */ {2, {10, 7, 0}, {1, 4, 0}, 0, 0, 0},
     /* 18 */ {2, {10, 8, 0}, {2, 3, 0}, 0, 0, 0},
     /* 19 */ {2, {8, 11, 0}, {4, 1, 0}, 1, 0, 0},
-    /* 20 */ {2, {12, 8, 0}, {1, 3, 0}, 1, 0, 1},
-    /* 21 */ {2, {11, 10, 0}, {1, 4, 0}, 0, 0, 1},
-    /* 22 */ {3, {8, 7, 7}, {3, 4, 4}, 1, 0, 1},
-    /* 23 */ {3, {8, 8, 7}, {3, 4, 4}, 1, 0, 1},
-    /* 24 */ {3, {8, 8, 8}, {3, 3, 3}, 0, 0, 1},
-    /* 25 */ {3, {8, 8, 9}, {3, 3, 3}, 0, 0, 1},
-    /* 26 */ {3, {8, 8, 10}, {3, 3, 3}, 0, 0, 1},
-    /* 27 */ {3, {8, 9, 10}, {4, 3, 3}, 0, 0, 1},
-    // 2^28 .. 2^30 (one 2^30 transform holds 16 GiB of buffers), timed among three-pass splits
-    // with default tile widths: 2^28 (10,10,8) 2.57 ms against (10,9,9) 2.62; 2^29 (10,10,9)
-    // 5.28 ms, the fastest of six; 2^30 (10,11,9) 11.2 ms against 12.6-16.2 ms for seven others,
-    // (10,10,10) 12.9 ms.
-    /* 28 */ {3, {10, 10, 8}, {3, 3, 4}, 1, 0, 1},
-    /* 29 */ {3, {10, 10, 9}, {3, 3, 4}, 1, 0, 1},
-    /* 30 */ {3, {10, 11, 9}, {3, 2, 4}, 1, 0, 1},
+    /* 20 */ {2, {12, 8, 0}, {1, 3, 0}, 1, 0, 0},
+    /* 21 */ {2, {11, 10, 0}, {1, 4, 0}, 0, 0, 0},
+    /* 22 */ {3, {8, 7, 7}, {3, 4, 4}, 1, 0, 0},
+    /* 23 */ {3, {8, 8, 7}, {3, 4, 4}, 1, 0, 0},
+    /* 24 */ {3, {8, 8, 8}, {3, 3, 3}, 0, 0, 0},
+    /* 25 */ {3, {8, 8, 9}, {3, 3, 3}, 0, 0, 0},
+    /* 26 */ {3, {8, 8, 10}, {3, 3, 3}, 0, 0, 0},
+    /* 27 */ {3, {8, 9, 10}, {4, 3, 3}, 0, 0, 0},
+    /* 28 */ {3, {10, 10, 8}, {3, 3, 4}, 1, 0, 0},
+    /* 29 */ {3, {10, 10, 9}, {3, 3, 4}, 1, 0, 0},
+    /* 30 */ {3, {10, 11, 9}, {3, 2, 4}, 1, 0, 0},
 };
-static_assert(sizeof(kTuned) / sizeof(kTuned[0]) == 30 - 15 + 1, "one shape per size 2^15 .. 2^30");
+static_assert(sizeof(kPlain) / sizeof(kPlain[0]) == 30 - 17 + 1, "one shape per size 2^17 .. 2^30");
+static const Shape *plain_shape(int m) { return m < 17 ? nullptr : &kPlain[m - 17]; }
 
 // Transforms per block (log2) of the one-kernel sizes 2^4 .. 2^14, from
 // `python -m onefft_b200.autotune --batched` on a B200 (forward, 2^25 values per batch, median of
@@ -208,7 +251,7 @@ static bool valid_shape(int m, const Shape &s) {
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-static onefft_plan *plan_build(size_t n, int m, const Shape &shape) {
+static onefft_plan *plan_build(size_t n, int m, const Shape &shape, const Shape *plain = nullptr) {
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) {
@@ -232,12 +275,29 @@ static onefft_plan *plan_build(size_t n, int m, const Shape &shape) {
         p->len[i] = shape.len[i];
         p->cols[i] = shape.cols[i];
     }
-    // layout: stage tables per pass, then the FP64 tables
-    size_t off[3], bytes = 0;
-    for (int i = 0; i < p->npass; ++i) {
-        off[i] = bytes;
-        bytes = align256(bytes + sizeof(float2) * (size_t)stage_table_entries_host(p->len[i]));
+    if (plain) {
+        p->plain_npass = plain->npass;
+        p->plain_l2_keep = plain->l2_keep;
+        for (int i = 0; i < plain->npass; ++i) {
+            p->plain_len[i] = plain->len[i];
+            p->plain_cols[i] = plain->cols[i];
+        }
     }
+    // layout: one stage table per pass length, then the FP64 tables
+    size_t table[13] = {}, bytes = 0;  // offsets by log2 length (passes), of the one-kernel sizes beyond
+    int tables[6], ntables = 0;   // the lengths, each once
+    size_t single_off = 0;
+    auto add_table = [&](int len) {
+        for (int i = 0; i < ntables; ++i)
+            if (tables[i] == len) return;
+        if (len <= 12) table[len] = bytes;
+        else single_off = bytes;
+        tables[ntables++] = len;
+        bytes = align256(bytes + sizeof(float2) * (size_t)stage_table_entries_host(len));
+    };
+    auto table_off = [&](int len) { return len <= 12 ? table[len] : single_off; };
+    for (int i = 0; i < p->npass; ++i) add_table(p->len[i]);
+    for (int i = 0; i < p->plain_npass; ++i) add_table(p->plain_len[i]);
     size_t lo_off = bytes, hi_off = bytes;
     if (p->npass >= 2) {
         p->lo_bits = m / 2;
@@ -281,10 +341,10 @@ static onefft_plan *plan_build(size_t n, int m, const Shape &shape) {
     cudaStream_t s = nullptr;
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
-        for (int i = 0; i < p->npass && e == cudaSuccess; ++i) {
-            p->stw[i] = (const float2 *)(base + off[i]);
-            e = launch_stage_table((float2 *)(base + off[i]), p->len[i], s);
-        }
+        for (int i = 0; i < p->npass; ++i) p->stw[i] = (const float2 *)(base + table_off(p->len[i]));
+        for (int i = 0; i < p->plain_npass; ++i) p->plain_stw[i] = (const float2 *)(base + table_off(p->plain_len[i]));
+        for (int i = 0; i < ntables && e == cudaSuccess; ++i)
+            e = launch_stage_table((float2 *)(base + table_off(tables[i])), tables[i], s);
         if (p->npass >= 2 && e == cudaSuccess) {
             p->tw_lo = (const double2 *)(base + lo_off);
             p->tw_hi = (const double2 *)(base + hi_off);
@@ -320,7 +380,7 @@ extern "C" onefft_plan *onefft_plan_create(size_t n) {
         set_error(ONEFFT_ERR_SIZE, "n=%zu is not a power of two in [1, 2^30]", n);
         return nullptr;
     }
-    return plan_build(n, m, tuned_shape(m));
+    return plan_build(n, m, tuned_shape(m), plain_shape(m));
 }
 
 extern "C" onefft_plan *onefft_plan_create_tiles(size_t n, int npass, const int *log2_len, const int *log2_cols,
@@ -363,6 +423,12 @@ extern "C" onefft_plan *onefft_plan_create_tiles(size_t n, int npass, const int 
 static const unsigned long long kBf16x3Accepted = 0;
 static const unsigned long long kBf16x6Accepted = ((1ull << 24) - 1) & ~((1ull << 4) - 1);  // 2^4 .. 2^23
 
+// Pass lengths (log2) of the split-BF16 plans of 2^15 .. 2^30: those their error bounds above were
+// measured with.
+static const int kBf16Len[16][3] = {{8, 7, 0},  {8, 8, 0},  {10, 7, 0}, {10, 8, 0}, {8, 11, 0},   {12, 8, 0},
+                                    {11, 10, 0}, {8, 7, 7}, {8, 8, 7},  {8, 8, 8},  {8, 8, 9},    {8, 8, 10},
+                                    {8, 9, 10}, {10, 10, 8}, {10, 10, 9}, {10, 11, 9}};
+
 static onefft_plan *create_bf16(size_t n, int terms, unsigned long long accepted, int require_accepted) {
     int m;
     if (!size_log2(n, &m) || m < 4) {
@@ -375,9 +441,13 @@ static onefft_plan *create_bf16(size_t n, int terms, unsigned long long accepted
         return nullptr;
     }
     Shape s = tuned_shape(m);
-    s.chunk = 0;
-    s.tma = 0;
-    s.fuse_lag = 0;
+    if (m > kMaxSingleLog2) {
+        const int *len = kBf16Len[m - 15];
+        s = Shape{};
+        s.npass = len[2] ? 3 : 2;
+        s.l2_keep = m == 19 || m == 20 || m == 22 || m == 23 || m >= 28;
+        for (int i = 0; i < s.npass; ++i) s.len[i] = len[i];
+    }
     for (int i = 0; i < s.npass; ++i) {
         s.cols[i] = pass_log_c(s.len[i]);
         if (s.npass > 1 && s.len[i] < 5) {
@@ -469,8 +539,10 @@ static cudaError_t plan_enqueue(const onefft_plan *p, const float2 *in, float2 *
     // pass i through its TMA kernel where the plan asks for it and the shape and buffers allow
     const bool use_tma = p->tma && !p->tc && batch <= 65535 && ((((uintptr_t)in | (uintptr_t)out) & 15) == 0);
     auto run = [&](int mode, int i, const PassArgs &x) {
-        if (use_tma && pass_tma_supported(p->len[i], p->cols[i]))
-            return launch_pass_tma(mode, p->len[i], p->cols[i], x, (int)batch, s);
+        const int wide = p->cols[i] & kWideTile, cols = p->cols[i] & ~kWideTile;
+        if (use_tma && wide) return launch_pass_wide(mode, p->len[i], cols, x, (int)batch, s);
+        if (use_tma && pass_tma_supported(p->len[i], cols))
+            return launch_pass_tma(mode, p->len[i], cols, x, (int)batch, s);
         return p->tc ? launch_pass_tc(mode, p->len[i], x, (int)batch, p->tc, s)
                      : launch_pass(mode, p->len[i], p->cols[i], x, (int)batch, s);
     };
@@ -575,26 +647,31 @@ static cudaError_t plan_enqueue(const onefft_plan *p, const float2 *in, float2 *
         g_launches.fetch_add(1);
         return run(2, 2, a);
     }
+    const bool plain = p->plain_npass && !use_tma;
+    const int npass = plain ? p->plain_npass : p->npass;
+    const int *len = plain ? p->plain_len : p->len;
+    if (plain) a.l2_keep = p->plain_l2_keep;
     int done = 0;  // log2 of the digits transformed so far
-    for (int i = 0; i < p->npass; ++i) {
-        const bool first = i == 0, last = i == p->npass - 1;
+    for (int i = 0; i < npass; ++i) {
+        const bool first = i == 0, last = i == npass - 1;
         a.in = first ? in : out;
         a.out = out;
-        a.stw = p->stw[i];
+        a.stw = plain ? p->plain_stw[i] : p->stw[i];
         a.swap_in = first && inverse;
         a.swap_out = last && inverse;
         if (first) {
-            a.log_s = p->log2n - p->len[0];
-            a.rev_b1 = p->len[1];
-            a.rev_b2 = p->npass == 3 ? p->len[2] : 0;
+            a.log_s = p->log2n - len[0];
+            a.rev_b1 = len[1];
+            a.rev_b2 = npass == 3 ? len[2] : 0;
         } else {
             a.log_s = done;
         }
         int mode = first ? 0 : last ? 2 : 1;
         g_launches.fetch_add(1);
-        cudaError_t e = run(mode, i, a);
+        cudaError_t e = plain ? launch_pass(mode, len[i], p->plain_cols[i], a, (int)batch, s)
+                              : run(mode, i, a);
         if (e != cudaSuccess) return e;
-        done += p->len[i];
+        done += len[i];
     }
     return cudaSuccess;
 }
