@@ -147,6 +147,9 @@ cudaError_t launch_pass_tma(int mode, int log_l, int log_c, const PassArgs& a, i
 // Wide-tile persistent passes (fft_wide.cu): same arithmetic, arguments and requirements as
 // launch_pass_tma (no chunks); the shapes the tuned table marks (onefft_api.cu, kWideTile)
 cudaError_t launch_pass_wide(int mode, int log_l, int log_c, const PassArgs& a, int batch, cudaStream_t stream);
+// A column-transform pass through its wide-tile kernel (as launch_pass_columns_tma; a.out 16-byte aligned)
+bool pass_columns_wide_supported(int mode, int log_l, const PassArgs& a);
+cudaError_t launch_pass_columns_wide(int mode, int log_l, const PassArgs& a, cudaStream_t stream);
 // split-BF16 tensor-core variants (fft_tc.cu) of `terms` = 3 or 6 split products: n = 2^4 .. 2^14
 // in one kernel; pass lengths 2^5 .. 2^12 with the default tile width pass_log_c()
 cudaError_t launch_single_kernel_tc(int log2n, const float2* in, float2* out, long long batch, const float2* stw,

@@ -124,7 +124,11 @@ __device__ __forceinline__ void pair_stages(float2 (&v)[2][16], int j, int c, in
     }
 }
 
-template <int LOG_L, int LOG_C, int MODE, bool SWAP, bool W>
+// SWAP: the first pass exchanges re/im on load, the last on store. W: weights (PassArgs::pre, post). X: a
+// pass of a column transform (PassArgs' column fields, as tma_tile; re/im exchanges at run time): the
+// tile of a.in, the column factors, and the first pass with colstore or the last pass writing the
+// column layout.
+template <int LOG_L, int LOG_C, int MODE, bool SWAP, bool W, bool X = false>
 __global__ void __launch_bounds__(Wide<LOG_L, LOG_C>::THREADS, LOG_L + LOG_C >= 14 ? 1 : LOG_L + LOG_C == 13 ? 2 : 4)
     k_pass_wide(PassArgs a, const __grid_constant__ CUtensorMap tin, unsigned tiles, int log_tiles) {
     using G = Wide<LOG_L, LOG_C>;
@@ -168,7 +172,15 @@ __global__ void __launch_bounds__(Wide<LOG_L, LOG_C>::THREADS, LOG_L + LOG_C >= 
         // two buffers, since slower threads may still read the previous tile's
         float2* tws = reinterpret_cast<float2*>(wide_smem + G::TW_OFF) + parity * (G::C * 17);
         float2 wl[2];
-        if (MODE != 2) {
+        bool twiddled = MODE != 2;
+        if constexpr (X) {
+            twiddled = a.tw_lo != nullptr;  // the same for the whole block
+            if (twiddled) {
+                column_twiddle_rows<LOG_L, LOG_C, MODE>(a, col0, tws, tid, G::THREADS);
+                wl[0] = column_twiddle_lane<LOG_L, MODE>(a, col0, 2 * cl, jl);
+                wl[1] = column_twiddle_lane<LOG_L, MODE>(a, col0, 2 * cl + 1, jl);
+            }
+        } else if (MODE != 2) {
             pass_twiddle_rows<LOG_L, LOG_C, MODE>(a, col0, tws, tid, G::THREADS);
             const unsigned f = MODE == 0 ? col0 + 2 * cl : (col0 >> a.log_s) << a.log_s;
             wl[0] = pass_twiddle_lane<LOG_L>(a, f, jl);
@@ -186,7 +198,7 @@ __global__ void __launch_bounds__(Wide<LOG_L, LOG_C>::THREADS, LOG_L + LOG_C >= 
                 if constexpr (W && MODE == 0) {
                     if (pre) v[i][k] = cmul(v[i][k], __ldg(pre + col0 + 2 * c + i + ((unsigned)(j + G::T * k) << a.log_s)));
                 }
-                if (SWAP && MODE == 0) v[i][k] = swap_ri(v[i][k]);
+                if (X ? a.swap_in : SWAP && MODE == 0) v[i][k] = swap_ri(v[i][k]);
             }
         }
         if (__syncthreads_or(!ok)) {
@@ -202,7 +214,7 @@ __global__ void __launch_bounds__(Wide<LOG_L, LOG_C>::THREADS, LOG_L + LOG_C >= 
             load(t + gridDim.x);
         }
         pair_stages<LOG_L, LOG_C, 0, MODE == 0>(v, j, c, jl, cl, a.stw, ex);
-        if (MODE != 2) {
+        if (twiddled) {
             const float2* tw = tws + (MODE == 0 ? 2 * cl * 17 : 0);
 #pragma unroll
             for (int k = 0; k < 16; ++k) {
@@ -210,7 +222,22 @@ __global__ void __launch_bounds__(Wide<LOG_L, LOG_C>::THREADS, LOG_L + LOG_C >= 
                 v[1][k] = cmul(v[1][k], cmul(wl[1], tw[MODE == 0 ? 17 + k : k]));
             }
         }
-        if (MODE == 0) {
+        // Column layout (column_dst), for blocks of at least the 16th part of the output's extent: output
+        // k + (16th part) i of transform b goes to its block's row b, i's part of the offset being the
+        // same for all threads.
+        const int log_part = LOG_L - 4 + (MODE == 0 ? 0 : a.log_s);
+        auto part = [&](int i) {
+            const unsigned long long k = (unsigned long long)i << log_part;
+            return ((k >> a.xlog_blk) << (a.xlog_cols + a.xlog_blk)) + (k & ((1ull << a.xlog_blk) - 1));
+        };
+        if (X && MODE == 0 && a.colstore) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                float2* q = a.out + ((unsigned long long)(col0 + 2 * cl + i) << a.xlog_blk) + jl;
+#pragma unroll
+                for (int k = 0; k < 16; ++k) q[part(k)] = a.swap_out ? swap_ri(v[i][k]) : v[i][k];
+            }
+        } else if (MODE == 0) {
             // contiguous column runs at their digit-reversed place, as k_pass
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
@@ -222,27 +249,28 @@ __global__ void __launch_bounds__(Wide<LOG_L, LOG_C>::THREADS, LOG_L + LOG_C >= 
         } else {
             const unsigned q0 = col0 & ((1u << a.log_s) - 1), h = col0 >> a.log_s;
             const unsigned base = q0 + 2 * c + (h << (a.log_s + LOG_L));
+            float2* qx = X ? a.out + ((unsigned long long)h << a.xlog_blk) + q0 + 2 * c + ((unsigned)j << a.log_s) : nullptr;
 #pragma unroll
             for (int k = 0; k < 16; ++k) {
                 const unsigned e = base + ((unsigned)(j + G::T * k) << a.log_s);
                 float2 y[2];
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
-                    y[i] = SWAP && MODE == 2 ? swap_ri(v[i][k]) : v[i][k];
+                    y[i] = (X ? a.swap_out : SWAP && MODE == 2) ? swap_ri(v[i][k]) : v[i][k];
                     if constexpr (W && MODE == 2) {
                         if (post) y[i] = cmul(y[i], __ldg(post + e + i));
                     }
                 }
-                *reinterpret_cast<float4*>(a.out + toff + e) = make_float4(y[0].x, y[0].y, y[1].x, y[1].y);
+                *reinterpret_cast<float4*>(X ? qx + part(k) : a.out + toff + e) = make_float4(y[0].x, y[0].y, y[1].x, y[1].y);
             }
         }
     }
 }
 
-template <int LOG_L, int LOG_C, int MODE, bool SWAP, bool W>
+template <int LOG_L, int LOG_C, int MODE, bool SWAP, bool W, bool X = false>
 static cudaError_t launch_wide_w(const PassArgs& a, int batch, cudaStream_t stream) {
     using G = Wide<LOG_L, LOG_C>;
-    auto kernel = k_pass_wide<LOG_L, LOG_C, MODE, SWAP, W>;
+    auto kernel = k_pass_wide<LOG_L, LOG_C, MODE, SWAP, W, X>;
     static std::atomic<unsigned long long> done{0};
     cudaError_t e = smem_limit((const void*)kernel, G::SMEM, done);
     if (e != cudaSuccess) return e;
@@ -259,7 +287,7 @@ static cudaError_t launch_wide_w(const PassArgs& a, int batch, cudaStream_t stre
         grid_of[dev & 63].store(grid, std::memory_order_relaxed);
     }
     CUtensorMap tin;
-    if (!make_map(&tin, MODE == 0 ? a.in : a.out, MODE, a.log2n, LOG_L, LOG_C, a.log_s, batch))
+    if (!make_map(&tin, MODE == 0 || X ? a.in : a.out, MODE, a.log2n, LOG_L, LOG_C, a.log_s, batch))
         return cudaErrorInvalidValue;
     const int log_tiles = a.log2n - LOG_L - LOG_C;
     const unsigned tiles = (unsigned)batch << log_tiles;
@@ -298,6 +326,40 @@ cudaError_t launch_pass_wide(int mode, int log_l, int log_c, const PassArgs& a, 
 #undef OFB_WIDE_CASE1
 #undef OFB_WIDE_CASE2
     return cudaErrorInvalidValue;
+}
+
+// ---- column transforms ----------------------------------------------------------------------------
+
+// Tile width (log2 columns) of a column-transform pass, -1: none.
+static constexpr int column_wide_log_c(int mode, int log_l) {
+    return log_l == 12 ? (mode == 0 ? 1 : 2) : log_l == 11 ? (mode == 0 ? 2 : 3) : log_l == 10 ? (mode == 0 ? 3 : 4)
+           : log_l == 9 ? 4 : log_l == 8 ? 5 : -1;
+}
+
+// Measured against k_pass_tma's column passes (B200, warm): 2^27 values, one pass of 2^8 .. 2^12 values
+// 456 -> 438, 484 -> 471, 520 -> 488, 572 -> 513, 619 -> 563 us; two passes 2^16 859 -> 785, 2^17
+// 956 -> 889, 2^18 933 -> 860, 2^19 1028 -> 942, 2^20 1001 -> 891 us; 2^24 values 66 -> 65 (2^10), 75 -> 69
+// (2^11), 82 -> 76 us (2^12). Columns of 2^8 and 2^9 values take tiles of 32 and 16 columns, which
+// leave SMs idle on small matrices (2^20 values 5.1 -> 5.9 us, 2^24 114 -> 116): from 2^25 values on.
+bool pass_columns_wide_supported(int mode, int log_l, const PassArgs& a) {
+    const int c = column_wide_log_c(mode, log_l);
+    return c >= 0 && (log_l >= 10 || a.log2n >= 25) && a.log2n >= log_l + c && (mode == 0 || a.log_s >= c) &&
+           (!a.colstore || a.xlog_blk >= log_l - 4 + (mode == 0 ? 0 : a.log_s)) && ((uintptr_t)a.out & 15) == 0;
+}
+
+cudaError_t launch_pass_columns_wide(int mode, int log_l, const PassArgs& a, cudaStream_t stream) {
+#define OFB_WIDE_COLUMNS(LL) \
+    case LL: return mode == 0 ? launch_wide_w<LL, column_wide_log_c(0, LL), 0, false, false, true>(a, 1, stream) \
+                              : launch_wide_w<LL, column_wide_log_c(2, LL), 2, false, false, true>(a, 1, stream);
+    switch (log_l) {
+        OFB_WIDE_COLUMNS(12)
+        OFB_WIDE_COLUMNS(11)
+        OFB_WIDE_COLUMNS(10)
+        OFB_WIDE_COLUMNS(9)
+        OFB_WIDE_COLUMNS(8)
+    default: return cudaErrorInvalidValue;
+    }
+#undef OFB_WIDE_COLUMNS
 }
 
 }  // namespace ofb

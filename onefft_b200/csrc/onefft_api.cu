@@ -1497,11 +1497,12 @@ extern "C" int onefft_columns_execute(const onefft_columns *c, const float *d_in
         return set_error(ONEFFT_ERR_ARG, "the column transform belongs to device %d, the current device is %d",
                          c->device, cur);
     const cudaStream_t s = (cudaStream_t)stream;
-    // a pass runs through its bulk-tensor-copy tile when its length has one and what it reads is
-    // 16-byte aligned (the work array always is)
+    // a pass runs through its wide or its one-per-block bulk-tensor-copy tile when its length has one
+    // and what it reads is 16-byte aligned (the work array always is)
     const bool in16 = ((uintptr_t)d_in & 15) == 0;
     auto run = [&](int mode, int len, const PassArgs &x, bool aligned) {
         g_launches.fetch_add(1);
+        if (aligned && pass_columns_wide_supported(mode, len, x)) return launch_pass_columns_wide(mode, len, x, s);
         if (aligned && column_tma_log_c(len) >= 0) return launch_pass_columns_tma(mode, len, x, s);
         return launch_pass_columns(mode, len, x, s);
     };

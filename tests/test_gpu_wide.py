@@ -63,6 +63,29 @@ def test_unaligned_buffers_take_the_plain_table(ofb, log2n, batch):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("ln,lcols,lblocks,lbig", [(8, 17, 3, 28), (9, 16, 2, 0), (10, 4, 0, 0), (10, 10, 3, 24), (11, 5, 7, 20),
+                                                   (11, 8, 1, 24), (12, 4, 4, 24), (12, 9, 0, 0), (13, 12, 5, 30), (16, 9, 4, 32),
+                                                   (19, 6, 3, 30), (20, 4, 0, 0), (20, 5, 4, 40)])
+def test_column_passes_same_bits_as_unaligned(ofb, ln, lcols, lblocks, lbig):
+    """Aligned buffers (wide tiles where the layout allows them: blocks of at least a 16th of a pass's
+    extent) against buffers at an odd complex offset, with every combination of the exchanges."""
+    import torch
+    values = 1 << (ln + lcols)
+    col0 = 2 << lcols if lbig else 0
+    c = ofb.Columns(1 << ln, 1 << lcols, 1 << lblocks, 1 << lbig if lbig else 0, col0 if lbig and 3 << (ln + lcols) <= 1 << lbig else 0)
+    x = torch.randn(2 * values, device="cuda", generator=torch.Generator(device="cuda").manual_seed(ln * 32 + lcols))
+    xs = torch.empty(2 * values + 2, device="cuda")[2:]
+    xs.copy_(x)
+    a, b = torch.empty_like(x), torch.empty(2 * values + 2, device="cuda")[2:]
+    stream = torch.cuda.current_stream().cuda_stream
+    for flags in (0, ofb.SWAP_IN, ofb.SWAP_OUT, ofb.SWAP_IN | ofb.SWAP_OUT):
+        c.execute(x.data_ptr(), a.data_ptr(), flags, stream)
+        c.execute(xs.data_ptr(), b.data_ptr(), flags, stream)
+        torch.cuda.synchronize()
+        c.check()
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("log2n", [18, 20, 24])
 def test_expired_wait_is_reported(ofb, log2n):
     import torch
