@@ -123,6 +123,7 @@ bool pass_tma_supported(int log_l, int log_c);
 cudaError_t set_expire_waits(int on);
 cudaError_t set_expire_waits_long(int on);  // fft_long.cu's part of it
 cudaError_t set_expire_waits_wide(int on);  // fft_wide.cu's
+cudaError_t set_expire_waits_cluster(int on);  // fft_cluster.cu's
 // Passes 0 and 1 of a three-pass transform (pass lengths 2^l0, 2^l1, 2^len2, tile widths 2^c0,
 // 2^c1) in ONE persistent launch over chunks of 2^g last-digit columns, pass 1 trailing pass 0 by
 // `lag` chunks (fft_tma.cu, k_pass01_fused). a0 / a1: the arguments of the chunked launches of
@@ -150,6 +151,10 @@ cudaError_t launch_pass_wide(int mode, int log_l, int log_c, const PassArgs& a, 
 // A column-transform pass through its wide-tile kernel (as launch_pass_columns_tma; a.out 16-byte aligned)
 bool pass_columns_wide_supported(int mode, int log_l, const PassArgs& a);
 cudaError_t launch_pass_columns_wide(int mode, int log_l, const PassArgs& a, cudaStream_t stream);
+// A batch of 2^15 in one launch, a transform per cluster of two blocks (fft_cluster.cu): the arithmetic
+// of the passes 2^8 and 2^7, same bits (a: in, out, tables and the first pass's stw; stw_b: the
+// second's); 16-byte aligned buffers, batch <= 65535
+cudaError_t launch_cluster(const PassArgs& a, const float2* stw_b, int inverse, long long batch, cudaStream_t stream);
 // split-BF16 tensor-core variants (fft_tc.cu) of `terms` = 3 or 6 split products: n = 2^4 .. 2^14
 // in one kernel; pass lengths 2^5 .. 2^12 with the default tile width pass_log_c()
 cudaError_t launch_single_kernel_tc(int log2n, const float2* in, float2* out, long long batch, const float2* stw,

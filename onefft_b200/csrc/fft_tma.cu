@@ -20,7 +20,8 @@ cudaError_t set_expire_waits(int on) {
     const int v = on ? 1 : 0;
     cudaError_t e = cudaMemcpyToSymbol(g_expire_waits, &v, sizeof v);
     if (e == cudaSuccess) e = set_expire_waits_long(v);
-    return e == cudaSuccess ? set_expire_waits_wide(v) : e;
+    if (e == cudaSuccess) e = set_expire_waits_wide(v);
+    return e == cudaSuccess ? set_expire_waits_cluster(v) : e;
 }
 
 // Blocks per SM that the register allocation must allow (0: the compiler chooses freely). Measured

@@ -23,6 +23,7 @@
 // FP64 work saves), stage twiddles loaded before the exchange that precedes their stage (no
 // change), strided last passes of 8 columns at strides of 512 KiB and more (64-byte pieces:
 // 2^27 1478 us against 1228 with 16 columns).
+#include "fft_pair.cuh"
 #include "fft_tma.cuh"
 
 namespace ofb {
@@ -51,32 +52,6 @@ struct Wide {
     static constexpr int BAR_OFF = TW_OFF + 2 * C * 17 * 8;
     static constexpr int SMEM = BAR_OFF + 16;
 };
-
-// Stage S on lane j of both columns (stage_compute, with each twiddle loaded once).
-template <int LOG_L, int S>
-__device__ __forceinline__ void pair_stage(float2 (&v)[2][16], int j, const float2* __restrict__ stw) {
-    using St = Stages<LOG_L>;
-    constexpr int LR = St::log2_radix(S), R = 1 << LR, NS = 1 << St::log2_ns(S), BPT = 16 / R;
-#pragma unroll
-    for (int i = 0; i < BPT; ++i) {
-        float2 a[2][R];
-#pragma unroll
-        for (int q = 0; q < R; ++q) a[0][q] = v[0][i + BPT * q], a[1][q] = v[1][i + BPT * q];
-        if (S > 0) {
-            const float2* tw = stw + St::tw_offset(S) + ((j + St::T * i) & (NS - 1));
-#pragma unroll
-            for (int q = 1; q < R; ++q) {
-                const float2 w = __ldg(tw + (q - 1) * NS);
-                a[0][q] = cmul(a[0][q], w);
-                a[1][q] = cmul(a[1][q], w);
-            }
-        }
-        dft<R>(a[0]);
-        dft<R>(a[1]);
-#pragma unroll
-        for (int p = 0; p < R; ++p) v[0][i + BPT * p] = a[0][p], v[1][i + BPT * p] = a[1][p];
-    }
-}
 
 // The exchange between stages S and S + 1 (tile_fft's): output p of lane j goes to element
 // E0(j) + p Ns of pair c, and element jr + T k of pair cr is read back, re and im parts one after

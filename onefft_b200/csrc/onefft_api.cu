@@ -105,6 +105,7 @@ struct onefft_plan {
     int tc;                // radix-16 stages as split-BF16 tensor-core products of this many terms (3: hi/lo,
                            // onefft_plan_create_bf16x3; 6: hi/mid/lo, onefft_plan_create_bf16x6); 0 = FP32
     int tma;               // passes staged through bulk tensor copies where the tile shape has a TMA kernel
+    int cluster_batch;     // batches of at least this many through the one-trip cluster kernel (0 = none)
     int fuse_lag;          // three passes, chunked: passes 0+1 as one persistent launch with pass 1
                            // trailing by this many chunks (0 = separate launches)
     unsigned *fused_ctr;   // kFusedSlots counter slots of fused_words words each, in `mem`
@@ -181,6 +182,11 @@ static const Shape kTuned[] = {
     /* 30 */ {3, {10, 10, 10}, {W(4), W(4), W(4)}, 0, 0, 1},
 };
 static_assert(sizeof(kTuned) / sizeof(kTuned[0]) == 30 - 15 + 1, "one shape per size 2^15 .. 2^30");
+
+// From this many transforms of 2^15 the cluster kernel (fft_cluster.cu; the same bits) is faster than
+// the two passes: five rounds of the 72 clusters a B200 holds (300 transforms 55 us in both, 160 40
+// against 29, 512 86 against 100).
+constexpr int kClusterBatch = 360;
 
 // The passes of calls whose buffers do not allow bulk tensor copies (not 16-byte aligned, or more
 // than 65535 transforms), 2^17 .. 2^30: per-thread loads run the long columns of the shapes above in
@@ -380,7 +386,9 @@ extern "C" onefft_plan *onefft_plan_create(size_t n) {
         set_error(ONEFFT_ERR_SIZE, "n=%zu is not a power of two in [1, 2^30]", n);
         return nullptr;
     }
-    return plan_build(n, m, tuned_shape(m), plain_shape(m));
+    onefft_plan *p = plan_build(n, m, tuned_shape(m), plain_shape(m));
+    if (p && m == 15) p->cluster_batch = kClusterBatch;
+    return p;
 }
 
 extern "C" onefft_plan *onefft_plan_create_tiles(size_t n, int npass, const int *log2_len, const int *log2_cols,
@@ -546,6 +554,13 @@ static cudaError_t plan_enqueue(const onefft_plan *p, const float2 *in, float2 *
         return p->tc ? launch_pass_tc(mode, p->len[i], x, (int)batch, p->tc, s)
                      : launch_pass(mode, p->len[i], p->cols[i], x, (int)batch, s);
     };
+    if (p->cluster_batch && batch >= p->cluster_batch && use_tma) {
+        a.in = in;
+        a.out = out;
+        a.stw = p->stw[0];
+        g_launches.fetch_add(1);
+        return launch_cluster(a, p->stw[1], inverse, batch, s);
+    }
     if (p->npass == 3 && p->fuse_lag && use_tma && !pre) {
         // Passes 0 and 1 in one persistent launch per transform (k_pass01_fused), then pass 2
         // over the batch. The launch needs a counter slot that no launch running at the same
