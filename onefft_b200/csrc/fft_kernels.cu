@@ -125,10 +125,12 @@ __global__ void __launch_bounds__(256) k_tiny(const float2* __restrict__ in, flo
 // padded layout the exchanges use (transform c's value e at spad(c n + e)). Measured on a B200
 // with 2^25 values per batch and 4096-value tiles, forward: n = 16 303 -> 90 us, n = 32 162 -> 94,
 // n = 64 104 -> 96 (82 us is the copy bound of the 537 MB moved); 2048-value tiles 86-87 us.
-template <int LOG_L, int LOG_C, int INV>
+// W: the weights pre / post, applied in registers, as batched_tile.
+template <int LOG_L, int LOG_C, int INV, bool W>
 __device__ __forceinline__ void batched_tile_staged(const float2* __restrict__ in, float2* __restrict__ out,
                                                     long long batch, const float2* __restrict__ stw, float2* smem,
-                                                    int tid) {
+                                                    int tid, const float2* __restrict__ pre,
+                                                    const float2* __restrict__ post) {
     constexpr int L = 1 << LOG_L, T = L / 16, THREADS = 1 << (LOG_L + LOG_C - 4);
     const long long g0 = (long long)blockIdx.x << LOG_C;
     const long long left = batch - g0;
@@ -146,7 +148,13 @@ __device__ __forceinline__ void batched_tile_staged(const float2* __restrict__ i
     {
         const float2* r = smem + spad(c * L + j);
 #pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = INV ? swap_ri(r[padc(k * T)]) : r[padc(k * T)];
+        for (int k = 0; k < 16; ++k) {
+            float2 x = r[padc(k * T)];
+            if constexpr (W) {
+                if (pre) x = cmul(x, __ldg(pre + j + T * k));
+            }
+            v[k] = INV ? swap_ri(x) : x;
+        }
     }
     __syncthreads();  // every input is in registers before the exchanges reuse the memory
     tile_fft<LOG_L, 1>(v, j, stw, smem, c << LOG_L);
@@ -154,7 +162,13 @@ __device__ __forceinline__ void batched_tile_staged(const float2* __restrict__ i
     {
         float2* w = smem + spad(c * L + j);
 #pragma unroll
-        for (int k = 0; k < 16; ++k) w[padc(k * T)] = INV ? swap_ri(v[k]) : v[k];
+        for (int k = 0; k < 16; ++k) {
+            float2 y = INV ? swap_ri(v[k]) : v[k];
+            if constexpr (W) {
+                if (post) y = cmul(y, __ldg(post + j + T * k));
+            }
+            w[padc(k * T)] = y;
+        }
     }
     __syncthreads();
 #pragma unroll
@@ -175,8 +189,8 @@ __global__ void __launch_bounds__(1 << (LOG_L + LOG_C - 4))
     dependent_launch();
     dependent_wait();
     if constexpr (W) pre = after_wait(pre), post = after_wait(post);
-    if constexpr (LOG_L <= 6 && !W) {
-        batched_tile_staged<LOG_L, LOG_C, INV>(in, out, batch, stw, smem, tid);
+    if constexpr (LOG_L <= 6) {
+        batched_tile_staged<LOG_L, LOG_C, INV, W>(in, out, batch, stw, smem, tid, pre, post);
     } else {
         const long long g = ((long long)blockIdx.x << LOG_C) + (tid >> (LOG_L - 4));
         batched_tile<LOG_L, LOG_C, false, W>(in + (g << LOG_L), out + (g << LOG_L), g < batch, INV, stw, smem, tid,
@@ -229,18 +243,24 @@ static cudaError_t launch_batched_w(const float2* in, float2* out, long long bat
     return cudaGetLastError();
 }
 
+template <int LOG_L, bool W>
+static cudaError_t launch_batched_c(const float2* in, float2* out, long long batch, const float2* stw, int inverse,
+                                    cudaStream_t stream, const float2* pre, const float2* post, int log_c) {
+    constexpr int B = default_batched_log_c(LOG_L);
+    if constexpr (B >= 1)
+        if (log_c == B - 1)
+            return launch_batched_w<LOG_L, W, B - 1>(in, out, batch, stw, inverse, stream, pre, post);
+    if constexpr (LOG_L + B + 1 <= 13)
+        if (log_c == B + 1)
+            return launch_batched_w<LOG_L, W, B + 1>(in, out, batch, stw, inverse, stream, pre, post);
+    return launch_batched_w<LOG_L, W, B>(in, out, batch, stw, inverse, stream, pre, post);
+}
+
 template <int LOG_L>
 static cudaError_t launch_batched_t(const float2* in, float2* out, long long batch, const float2* stw, int inverse,
                                     cudaStream_t stream, const float2* pre, const float2* post, int log_c) {
-    constexpr int B = default_batched_log_c(LOG_L);
-    if (pre || post) return launch_batched_w<LOG_L, true, B>(in, out, batch, stw, inverse, stream, pre, post);
-    if constexpr (B >= 1)
-        if (log_c == B - 1)
-            return launch_batched_w<LOG_L, false, B - 1>(in, out, batch, stw, inverse, stream, nullptr, nullptr);
-    if constexpr (LOG_L + B + 1 <= 13)
-        if (log_c == B + 1)
-            return launch_batched_w<LOG_L, false, B + 1>(in, out, batch, stw, inverse, stream, nullptr, nullptr);
-    return launch_batched_w<LOG_L, false, B>(in, out, batch, stw, inverse, stream, nullptr, nullptr);
+    if (pre || post) return launch_batched_c<LOG_L, true>(in, out, batch, stw, inverse, stream, pre, post, log_c);
+    return launch_batched_c<LOG_L, false>(in, out, batch, stw, inverse, stream, nullptr, nullptr, log_c);
 }
 
 template <int LOG_N>

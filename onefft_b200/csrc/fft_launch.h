@@ -101,8 +101,7 @@ int pass_log_c(int log_l);
 bool pass_tile_supported(int log_l, int log_c);
 
 // pre / post: optional pointwise weights of the input and output (n complex values each);
-// log_c: transforms per block of k_batched (batched_log_c_supported; < 0 = the default; weighted
-// calls always use the default)
+// log_c: transforms per block of k_batched (batched_log_c_supported; < 0 = the default)
 cudaError_t launch_single_kernel(int log2n, const float2* in, float2* out, long long batch, const float2* stw,
                                  int inverse, cudaStream_t stream, const float2* pre = nullptr,
                                  const float2* post = nullptr, int log_c = -1);

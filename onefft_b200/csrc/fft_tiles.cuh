@@ -205,13 +205,15 @@ __device__ __forceinline__ void batched_tile(const float2* __restrict__ src, flo
     dst += j;
     float2 v[16];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-        float2 x = active ? ld_stream(src + T * k) : make_float2(0.f, 0.f);
-        if constexpr (W) {
-            if (pre) x = cmul(x, __ldg(pre + j + T * k));
+    for (int k = 0; k < 16; ++k) v[k] = active ? ld_stream(src + T * k) : make_float2(0.f, 0.f);
+    if constexpr (W) {  // after all loads: a test of `pre` between them would keep them apart
+        if (pre) {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] = cmul(v[k], __ldg(pre + j + T * k));
         }
-        v[k] = inverse ? swap_ri(x) : x;
     }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = inverse ? swap_ri(v[k]) : v[k];
     if constexpr (TC != 0) tile_fft_tc<LOG_L, LOG_C, 1, TC>(v, j, stw, smem, c << LOG_L, tid);
     else tile_fft<LOG_L, 1>(v, j, stw, smem, c << LOG_L);
     if (active) {
