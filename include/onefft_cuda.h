@@ -137,9 +137,9 @@ ONEFFT_API int onefft_plan_passes(const onefft_plan *plan, int *log2_len);
 /* ---- uneven batches ----------------------------------------------------------------------------
  * Counterpart of a caller looping over OneFFT's onefft_plan_forward/_inverse with a different
  * plan per size (src/onefft.c:1138-1140): many transforms of different power-of-two sizes packed
- * in one buffer, run by ONE persistent kernel launch that pulls work from a device queue. The
- * counter reset and the launch form a CUDA graph built by onefft_uneven_create() and replayed by
- * each execute. Transform i has size 2^log2n (0 <= log2n <= 16), starts at complex offset
+ * in one buffer, run by ONE persistent kernel launch that pulls work from a device queue and
+ * leaves its counters reset: a CUDA graph built by onefft_uneven_create() and replayed by each
+ * execute, or, beyond 2^16 values, a plain launch of the same kernel. Transform i has size 2^log2n (0 <= log2n <= 16), starts at complex offset
  * `offset` of both buffers, and runs forward (inverse = 0) or inverse (inverse = 1). Transforms
  * must not overlap each other. */
 typedef struct onefft_desc {

@@ -17,8 +17,9 @@
 //     transforms in flight, and the values between their passes stay in L2, where one block per
 //     transform kept hundreds of megabytes of them in flight. (With no unit queue, as in
 //     onefft_uneven_execute_noalloc, every block runs whole transforms; the same bits either way.)
-//   - the memset of the counter plus the launch form a CUDA graph built at creation; execute
-//     patches the buffer pointers into the kernel node and replays it.
+//   - the launch is a CUDA graph built at creation, replayed by execute with the buffer pointers
+//     patched in, or for batches beyond 2^16 values the same kernel as a dependent launch. The last
+//     block to leave zeroes the counters for the next launch.
 // Per work item the arithmetic is the plain path's tile body (fft_tiles.cuh) with the plain
 // path's tables, so results equal onefft_dev_*_batched of each transform bit for bit wherever
 // the split is the same (every size except 2^13 and 2^14, which the plain path runs as one
@@ -262,6 +263,7 @@ __global__ void __launch_bounds__(kUnevenThreads, 4) k_uneven(UnevenArgs a) {
     __shared__ int s_item;
     const int tid = threadIdx.x;
     const int count = a.units ? a.nunits : a.nitems;
+    dependent_wait();
     if (tid == 0) s_item = atomicAdd(a.counter, 1);
     __syncthreads();
     int s = s_item;
@@ -311,6 +313,20 @@ __global__ void __launch_bounds__(kUnevenThreads, 4) k_uneven(UnevenArgs a) {
         default: break;
         }
         __syncthreads();  // the next item may reuse shared memory
+    }
+    // The last block to leave zeroes the counters for the next launch (a memset node before the
+    // kernel cost small batches more than their transforms): every other block has left its loop, so
+    // none touches them again.
+    if (a.left) {
+        if (tid == 0) {
+            __threadfence();
+            s_item = atomicAdd(a.left, 1u) == gridDim.x - 1;
+        }
+        __syncthreads();
+        if (s_item) {
+            for (int k = tid; k <= a.nitems; k += kUnevenThreads) a.done[k] = 0;
+            if (tid == 0) *a.counter = 0, *a.left = 0;
+        }
     }
 }
 

@@ -62,13 +62,14 @@ struct UnevenArgs {
     const onefft_desc *desc;  // sorted copy of the descriptors
     const UnevenItem *items;
     int nitems;
-    int *counter;  // work queue head, zeroed before every launch
+    int *counter;  // work queue head, zero before every launch
     // Step-wise queue (NULL: every block runs whole items, the transforms of 2^13 .. 2^16 tile
     // after tile in one block): the units in queue order, and per item the pass-0 steps done,
-    // followed by one abort word (all zeroed before every launch, like the counter).
+    // followed by one abort word (all zero before every launch, like the counter).
     const UnevenUnit *units;
     int nunits;
     unsigned *done;
+    unsigned *left;  // blocks that have left; the last one zeroes all counters again (NULL: the caller does)
     unsigned *err;  // set when a pass-1 unit's bounded wait for its pass 0 ran out
     const float2 *stw[kUnevenMaxLog2 + 1][2];  // stage tables: [m][0] single kernel / pass 0, [m][1] pass 1
     const double2 *tw_lo[kUnevenMaxLog2 + 1];
