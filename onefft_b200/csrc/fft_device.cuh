@@ -278,4 +278,45 @@ __device__ __forceinline__ void tile_fft(float2 (&v)[16], int j, const float2* _
     }
 }
 
+// tile_fft of C = 2^LOG_C interleaved columns (COUNT >= 2 stages) whose last exchange regroups the
+// threads: on entry the thread holds lane j of column c (consecutive threads on consecutive columns),
+// on exit lane jl of column cl (consecutive threads along a column), so that a first pass stores
+// contiguous runs straight from registers instead of transposing its results through shared memory
+// once more. That exchange keeps whole columns [c][e], padded one slot every 16 and offset by 16 / C
+// slots a column: the writers (16 / C lanes of each column) and the readers (16 values of one
+// column) of a half-warp both meet 16 distinct banks. Against the extra transposition (two of the
+// tile's ten shared-memory accesses a value, and a barrier), warm, same bits: 256 x 2^16 99.5 -> 96.9 us,
+// 300 x 2^15 59 -> 56, one 2^25 299 -> 288, the uneven mix of 20000 1090 -> 1023, 300 uneven transforms of
+// 2^13 .. 2^16 72 -> 66.
+__host__ __device__ constexpr int regroup_column(int log_l, int log_c) {
+    return (1 << log_l) + (1 << (log_l - 4)) + (log_c <= 4 ? 16 >> log_c : 1);
+}
+// Slots of the exchange memory of such a tile (float2 units).
+__host__ __device__ constexpr int regroup_slots(int log_l, int log_c) { return regroup_column(log_l, log_c) << log_c; }
+
+template <int LOG_L, int LOG_C, int S = 0>
+__device__ __forceinline__ void tile_fft_regroup(float2 (&v)[16], int j, int c, int jl, int cl,
+                                                 const float2* __restrict__ stw, float2* smem) {
+    using St = Stages<LOG_L>;
+    static_assert(St::COUNT >= 2, "no exchange to regroup in");
+    constexpr int C = 1 << LOG_C;
+    constexpr bool LAST = S + 1 == St::COUNT;
+    stage_compute<LOG_L, S>(v, LAST ? jl : j, stw);
+    if constexpr (!LAST) {
+        constexpr int LNS = St::log2_ns(S), NS = 1 << LNS;
+        constexpr bool TO_LAST = S + 2 == St::COUNT;
+        const int e0 = ((j >> LNS) << (4 + LNS)) + (j & (NS - 1));
+        constexpr int LM = TO_LAST ? 1 : C;  // distance of consecutive elements, before padding
+        float2* w = TO_LAST ? smem + c * regroup_column(LOG_L, LOG_C) + spad(e0) : smem + spad(e0 * C + c);
+        const float2* r = TO_LAST ? smem + cl * regroup_column(LOG_L, LOG_C) + spad(jl) : smem + spad(j * C + c);
+#pragma unroll
+        for (int p = 0; p < 16; ++p) w[padc(p * NS * LM)] = v[p];
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = r[padc(k * St::T * LM)];
+        if constexpr (!TO_LAST) __syncthreads();
+        tile_fft_regroup<LOG_L, LOG_C, S + 1>(v, j, c, jl, cl, stw, smem);
+    }
+}
+
 }  // namespace ofb

@@ -401,7 +401,7 @@ template <int LOG_L, int MODE>
 static cudaError_t launch_columns_t(const PassArgs& a, cudaStream_t stream) {
     constexpr int LOG_C = default_pass_log_c(LOG_L);
     constexpr int THREADS = 1 << (LOG_L + LOG_C - 4);
-    constexpr int SMEM = pass_smem_bytes(LOG_L, LOG_C, 1);
+    constexpr int SMEM = pass_smem_bytes(LOG_L, LOG_C, MODE == 0 ? 0 : 1);  // factors in both modes
     auto kernel = k_pass<LOG_L, LOG_C, MODE, false, true>;
     static std::atomic<unsigned long long> done{0};
     const cudaError_t attr = smem_limit((const void*)kernel, SMEM, done);

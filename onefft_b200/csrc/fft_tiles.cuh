@@ -152,9 +152,15 @@ __device__ __forceinline__ bool wait_count_or_abort(const unsigned* p, unsigned 
 __host__ __device__ constexpr int smem_bytes(int log_l, int log_c) {
     return (int)sizeof(float2) * ((1 << (log_l + log_c)) + (1 << (log_l + log_c - 4)));
 }
-// ... plus the inter-pass twiddle factors of a pass tile (17 per column).
+// Slots (float2) of a pass tile's exchange memory: a first pass of two or more stages regroups its
+// threads in its last exchange (tile_fft_regroup).
+__host__ __device__ constexpr bool pass_regroups(int log_l, int mode) { return mode == 0 && log_l > 4; }
+__host__ __device__ constexpr int pass_slots(int log_l, int log_c, int mode) {
+    return pass_regroups(log_l, mode) ? regroup_slots(log_l, log_c) : (1 << (log_l + log_c)) + (1 << (log_l + log_c - 4));
+}
+// Shared memory of a pass tile: the exchange memory plus the inter-pass twiddle factors (17 per column).
 __host__ __device__ constexpr int pass_smem_bytes(int log_l, int log_c, int mode) {
-    return smem_bytes(log_l, log_c) + (mode == 2 ? 0 : (int)sizeof(float2) * 17 * (1 << log_c));
+    return (int)sizeof(float2) * (pass_slots(log_l, log_c, mode == 2 ? 2 : 0) + (mode == 2 ? 0 : 17 * (1 << log_c)));
 }
 
 // ---- n <= 8: one transform per thread -------------------------------------------------------------
@@ -264,18 +270,21 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, unsigned t, long lo
     // w^(F T kk) of each column in shared memory (rows padded to 17 so the columns of a warp hit
     // distinct banks), w^(F j) per thread; each rounded once to FP32, their product applied in
     // FP32 (pass_twiddle_rows / pass_twiddle_lane).
-    float2* tws = smem + spad(C * L - 1) + 1;
+    // REGROUP: after the last exchange the thread holds lane jl of column cl.
+    constexpr bool REGROUP = pass_regroups(LOG_L, MODE) && TC == 0;
+    const int cl = REGROUP ? tid >> (LOG_L - 4) : c, jl = REGROUP ? tid & (T - 1) : j;
+    float2* tws = smem + pass_slots(LOG_L, LOG_C, MODE);
     float2 wjf = make_float2(1.f, 0.f);
     bool twiddled = MODE != 2;
     if constexpr (X) {
         twiddled = MODE != 1 && a.tw_lo != nullptr;  // the same for the whole block
         if (twiddled) {
             column_twiddle_rows<LOG_L, LOG_C, MODE>(a, col0, tws, tid, C * T);
-            wjf = column_twiddle_lane<LOG_L, MODE>(a, col0, c, j);
+            wjf = column_twiddle_lane<LOG_L, MODE>(a, col0, cl, jl);
         }
     } else if (MODE != 2) {
         pass_twiddle_rows<LOG_L, LOG_C, MODE>(a, col0, tws, tid, C * T);
-        wjf = pass_twiddle_lane<LOG_L>(a, MODE == 0 ? col0 + c : (col0 >> a.log_s) << a.log_s, j);
+        wjf = pass_twiddle_lane<LOG_L>(a, MODE == 0 ? col0 + cl : (col0 >> a.log_s) << a.log_s, jl);
     }
     dependent_wait();  // (returns at once in the uneven kernel, whose launches are not dependent ones)
     const float2 *pre = nullptr, *post = nullptr;
@@ -297,43 +306,42 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, unsigned t, long lo
         }
     }
     if constexpr (TC != 0) tile_fft_tc<LOG_L, LOG_C, C, TC>(v, j, a.stw, smem, c, tid);
+    else if constexpr (REGROUP) tile_fft_regroup<LOG_L, LOG_C>(v, j, c, jl, cl, a.stw, smem);
     else tile_fft<LOG_L, C>(v, j, a.stw, smem, c);
     if (twiddled) {
         if (Stages<LOG_L>::COUNT == 1) __syncthreads();  // tile_fft had no barrier to publish tws
-        const float2* tw = tws + (MODE == 0 ? c * 17 : 0);
+        const float2* tw = tws + (MODE == 0 ? cl * 17 : 0);
 #pragma unroll
         for (int k = 0; k < 16; ++k) v[k] = cmul(v[k], cmul(wjf, tw[k]));
     }
     const unsigned long long keep = a.l2_keep ? policy_evict_last() : 0ull;
     if (MODE == 0) {
-        // Transpose through shared memory so that each column's L results leave as one
-        // contiguous, coalesced run: thread tid then stores values kk0 + T i (i = 0..15) of
-        // column cc = tid / T, at its digit-reversed place.
-        {
+        // Each column's L results leave as one contiguous, coalesced run at its digit-reversed place:
+        // thread tid stores values kk0 + T i (i = 0..15) of column cc = tid / T, which it holds
+        // (REGROUP) or gets through shared memory.
+        const int cc = tid >> (LOG_L - 4), kk0 = tid & (T - 1);
+        if constexpr (!REGROUP) {
             float2* w = smem + spad(j * C + c);
 #pragma unroll
             for (int k = 0; k < 16; ++k) w[padc(k * T * C)] = v[k];
-        }
-        __syncthreads();
-        const int cc = tid >> (LOG_L - 4), kk0 = tid & (T - 1);
-        const unsigned rr = col0 + cc;
-        if (X && a.colstore) {
+            __syncthreads();
             const float2* r = smem + spad(kk0 * C + cc);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const float2 x = r[padc(i * T * C)];
-                a.out[column_dst(a, rr, (unsigned)(kk0 + i * T))] = a.swap_out ? swap_ri(x) : x;
-            }
+            for (int i = 0; i < 16; ++i) v[i] = r[padc(i * T * C)];
+        }
+        const unsigned rr = col0 + cc;
+        if (X && a.colstore) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                a.out[column_dst(a, rr, (unsigned)(kk0 + i * T))] = a.swap_out ? swap_ri(v[i]) : v[i];
             return;
         }
         const unsigned j2 = rr & ((1u << a.rev_b2) - 1), j1 = rr >> a.rev_b2;
         float2* q = a.out + toff + (((j1 + (j2 << a.rev_b1)) << LOG_L) + kk0);
-        const float2* r = smem + spad(kk0 * C + cc);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            float2 x = r[padc(i * T * C)];
-            if (a.l2_keep) st_policy(q + i * T, x, keep);
-            else q[i * T] = x;
+            if (a.l2_keep) st_policy(q + i * T, v[i], keep);
+            else q[i * T] = v[i];
         }
     } else if (X && MODE == 2) {
         const unsigned long long h = col0 >> a.log_s, q = (col0 & ((1u << a.log_s) - 1)) + c;

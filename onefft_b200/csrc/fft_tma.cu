@@ -43,7 +43,7 @@ constexpr int tma_min_blocks() {
 // reused padded by the exchanges), the inter-pass twiddle factors (17 per column); the block's
 // mbarrier follows at this offset.
 __host__ __device__ constexpr int tma_bar_offset(int log_l, int log_c) {
-    return (1 << (log_l + log_c)) + (1 << (log_l + log_c - 4)) + 17 * (1 << log_c);
+    return pass_slots(log_l, log_c, 0) + 17 * (1 << log_c);
 }
 __host__ __device__ constexpr int tma_smem_bytes(int log_l, int log_c) {
     return (int)sizeof(float2) * (tma_bar_offset(log_l, log_c) + 2) + 16;
@@ -108,19 +108,22 @@ __device__ __forceinline__ bool tma_tile(const PassArgs& a, const CUtensorMap* t
             issued();
         }
     }
-    // inter-pass twiddle factors (as pass_tile) while the copy is in flight
-    float2* tws = smem + spad(C * L - 1) + 1;
+    // inter-pass twiddle factors (as pass_tile) while the copy is in flight; the first pass ends on lane
+    // jl of column cl (tile_fft_regroup)
+    constexpr bool REGROUP = pass_regroups(LOG_L, MODE);
+    const int cl = REGROUP ? tid >> (LOG_L - 4) : c, jl = REGROUP ? tid & (T - 1) : j;
+    float2* tws = smem + pass_slots(LOG_L, LOG_C, 0);
     float2 wjf = make_float2(1.f, 0.f);
     bool twiddled = MODE != 2;
     if constexpr (X) {
         twiddled = MODE != 1 && a.tw_lo != nullptr;  // the same for the whole block
         if (twiddled) {
             column_twiddle_rows<LOG_L, LOG_C, MODE>(a, col0, tws, tid, C * T);
-            wjf = column_twiddle_lane<LOG_L, MODE>(a, col0, c, j);
+            wjf = column_twiddle_lane<LOG_L, MODE>(a, col0, cl, jl);
         }
     } else if (MODE != 2) {
         pass_twiddle_rows<LOG_L, LOG_C, MODE>(a, col0, tws, tid, C * T);
-        wjf = pass_twiddle_lane<LOG_L>(a, MODE == 0 ? col0 + c : (col0 >> a.log_s) << a.log_s, j);
+        wjf = pass_twiddle_lane<LOG_L>(a, MODE == 0 ? col0 + cl : (col0 >> a.log_s) << a.log_s, jl);
     }
     // the barrier is initialised (and armed) before anyone waits on it
     if (__syncthreads_or(!go)) return false;  // nothing was issued: nothing to wait for
@@ -149,42 +152,33 @@ __device__ __forceinline__ bool tma_tile(const PassArgs& a, const CUtensorMap* t
         v[k] = a.swap_in ? swap_ri(x) : x;
     }
     __syncthreads();  // the dense tile is consumed; the exchanges reuse its memory
-    tile_fft<LOG_L, C>(v, j, a.stw, smem, c);
+    if constexpr (REGROUP) tile_fft_regroup<LOG_L, LOG_C>(v, j, c, jl, cl, a.stw, smem);
+    else tile_fft<LOG_L, C>(v, j, a.stw, smem, c);
     if (twiddled) {
         if (Stages<LOG_L>::COUNT == 1) __syncthreads();
-        const float2* tw = tws + (MODE == 0 ? c * 17 : 0);
+        const float2* tw = tws + (MODE == 0 ? cl * 17 : 0);
 #pragma unroll
         for (int k = 0; k < 16; ++k) v[k] = cmul(v[k], cmul(wjf, tw[k]));
     }
     if (MODE == 0) {
-        // contiguous column runs at their digit-reversed place, as k_pass
-        {
-            float2* w = smem + spad(j * C + c);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) w[padc(k * T * C)] = v[k];
-        }
-        __syncthreads();
-        const int cc = tid >> (LOG_L - 4), kk0 = tid & (T - 1);
-        const unsigned rr = col0 + cc;
+        // contiguous column runs at their digit-reversed place, as k_pass, straight from registers
+        static_assert(MODE != 0 || REGROUP, "every first-pass tile has an exchange to regroup in");
+        const unsigned rr = col0 + cl;
         if (X && a.colstore) {
-            const float2* r = smem + spad(kk0 * C + cc);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const float2 x = r[padc(i * T * C)];
-                a.out[column_dst(a, rr, (unsigned)(kk0 + i * T))] = a.swap_out ? swap_ri(x) : x;
-            }
+            for (int i = 0; i < 16; ++i)
+                a.out[column_dst(a, rr, (unsigned)(jl + i * T))] = a.swap_out ? swap_ri(v[i]) : v[i];
             return true;
         }
         const unsigned j2 = rr & ((1u << a.rev_b2) - 1), j1 = rr >> a.rev_b2;
-        float2* q = a.out + ((long long)b << a.log2n) + (((j1 + (j2 << a.rev_b1)) << LOG_L) + kk0);
-        const float2* r = smem + spad(kk0 * C + cc);
+        float2* q = a.out + ((long long)b << a.log2n) + (((j1 + (j2 << a.rev_b1)) << LOG_L) + jl);
         if (a.l2_keep) {
             const unsigned long long keep = policy_evict_last();  // the next pass reads these
 #pragma unroll
-            for (int i = 0; i < 16; ++i) st_policy(q + i * T, r[padc(i * T * C)], keep);
+            for (int i = 0; i < 16; ++i) st_policy(q + i * T, v[i], keep);
         } else {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) q[i * T] = r[padc(i * T * C)];
+            for (int i = 0; i < 16; ++i) q[i * T] = v[i];
         }
     } else if (X && MODE == 2) {
         const unsigned long long hh = (unsigned)h, q = (unsigned)(q0 + c);
