@@ -283,9 +283,9 @@ static cudaError_t launch_wide_t(const PassArgs& a, int batch, cudaStream_t stre
 }
 
 // Tile shapes (log2 values, log2 columns) with a wide kernel, by pass: those the tuned table uses.
-#define OFB_WIDE_FIRST(X) X(12, 1) X(11, 2) X(10, 4) X(10, 3) X(9, 4) X(8, 5)
-#define OFB_WIDE_MIDDLE(X) X(10, 4) X(9, 4) X(8, 5)
-#define OFB_WIDE_LAST(X) X(12, 2) X(11, 3) X(10, 4) X(10, 3) X(9, 4) X(8, 4)
+#define OFB_WIDE_FIRST(X) X(12, 1) X(11, 2) X(10, 4) X(10, 3) X(9, 4)
+#define OFB_WIDE_MIDDLE(X) X(10, 4) X(9, 4)
+#define OFB_WIDE_LAST(X) X(12, 2) X(11, 3) X(10, 4) X(10, 3) X(8, 4)
 
 cudaError_t launch_pass_wide(int mode, int log_l, int log_c, const PassArgs& a, int batch, cudaStream_t stream) {
 #define OFB_WIDE_CASE0(LL, LC) \

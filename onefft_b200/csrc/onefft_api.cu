@@ -158,10 +158,12 @@ struct Shape {
 //   2^22 (8,7,7)   35.4 / 99.9 (3)  / 281 (8)    -> 36.3 / 95.9 / 231
 //   2^23 (8,8,7)   62.6 /             288 (4)    -> 67.5 /        240
 //   2^24 (8,8,8)   143  /             281 (2)    -> 132  /        254
-//   2^26 (8,8,10)  586 -> 575;  2^27 (8,9,10) 1228 -> 1155;  2^28 (10,10,8) 2702 -> (9,9,10) 2408;
-//   2^29 (10,10,9) 5534 -> (9,10,10) 5162;  2^30 (10,11,9) 11499 -> (10,10,10) 10571
-// 2^15, 2^16 and 2^25 keep k_pass_tma: no wide shape was faster (2^16 in (8,8), also the split of the
-// uneven batch's in-block passes, which stay bit-identical to this path).
+//   2^28 (10,10,8) 2702 -> (9,9,10) 2408;  2^29 (10,10,9) 5534 -> (9,10,10) 5162;
+//   2^30 (10,11,9) 11499 -> (10,10,10) 10571
+// 2^15, 2^16 and 2^25 .. 2^27 keep k_pass_tma. No wide shape was faster at 2^15, 2^16 (in (8,8), also
+// the split of the uneven batch's in-block passes, which stay bit-identical to this path) and 2^25.
+// At 2^26 and 2^27 wide shapes gain 1-2 % where the power limit holds the clock down (2^27 1192 .. 1213 us
+// against 1224) and lose 6-7 % in short runs at the full clock (1101 .. 1109 against 1035).
 constexpr int W(int c) { return kWideTile | c; }
 static const Shape kTuned[] = {
     /* 15 */ {2, {8, 7, 0}, {3, 4, 0}, 0, 0, 1},
@@ -175,8 +177,8 @@ static const Shape kTuned[] = {
     /* 23 */ {2, {12, 11, 0}, {W(1), W(3), 0}, 0, 0, 1},
     /* 24 */ {2, {12, 12, 0}, {W(1), W(2), 0}, 0, 0, 1},
     /* 25 */ {3, {8, 8, 9}, {3, 3, 3}, 0, 0, 1},
-    /* 26 */ {3, {9, 8, 9}, {W(4), W(5), W(4)}, 0, 0, 1},
-    /* 27 */ {3, {8, 9, 10}, {W(5), W(4), W(4)}, 0, 0, 1},
+    /* 26 */ {3, {8, 8, 10}, {4, 3, 3}, 0, 0, 1},
+    /* 27 */ {3, {8, 9, 10}, {4, 3, 3}, 0, 0, 1},
     /* 28 */ {3, {9, 9, 10}, {W(4), W(4), W(4)}, 0, 0, 1},
     /* 29 */ {3, {9, 10, 10}, {W(4), W(4), W(4)}, 0, 0, 1},
     /* 30 */ {3, {10, 10, 10}, {W(4), W(4), W(4)}, 0, 0, 1},

@@ -1,4 +1,4 @@
-"""GPU tests of the wide-tile passes (csrc/fft_wide.cu), which the tuned table uses from 2^18 on.
+"""GPU tests of the wide-tile passes (csrc/fft_wide.cu), which the tuned table uses at 2^18 .. 2^24 and 2^28 .. 2^30.
 
 They do the arithmetic of the per-thread-load passes (k_pass) on the same values, so a default plan
 gives the bits of a plan with the same pass lengths and no bulk copies: both directions, with either
@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 # size -> (pass lengths of the default plan, pass lengths for unaligned buffers)
 SPLITS = {17: ((8, 9), (10, 7)), 18: ((10, 8), (10, 8)), 19: ((11, 8), (8, 11)), 20: ((10, 10), (12, 8)),
           21: ((11, 10), (11, 10)), 22: ((11, 11), (8, 7, 7)), 23: ((12, 11), (8, 8, 7)), 24: ((12, 12), (8, 8, 8)),
-          26: ((9, 8, 9), (8, 8, 10)), 27: ((8, 9, 10), (8, 9, 10)), 28: ((9, 9, 10), (10, 10, 8))}
+          26: ((8, 8, 10), (8, 8, 10)), 27: ((8, 9, 10), (8, 9, 10)), 28: ((9, 9, 10), (10, 10, 8))}
 CASES = [(17, 9), (18, 1), (18, 7), (19, 1), (19, 5), (20, 1), (20, 3), (21, 1), (21, 3), (22, 1), (22, 2), (23, 1),
          (24, 1), (24, 2), (26, 1), (27, 1), (28, 1)]
 
