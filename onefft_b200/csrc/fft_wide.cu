@@ -21,8 +21,8 @@
 //
 // Measured and left out: inter-pass powers shared by the block (the extra latency costs what the
 // FP64 work saves), stage twiddles loaded before the exchange that precedes their stage (no
-// change), strided last passes of 8 columns at strides of 512 KiB and more (64-byte pieces:
-// 2^27 1478 us against 1228 with 16 columns).
+// change), strided last passes of 8 columns at strides of 512 KiB and more (64-byte pieces: 2^27
+// 1478 us; 1213 with 16 columns).
 #include "fft_pair.cuh"
 #include "fft_tma.cuh"
 
@@ -305,17 +305,18 @@ cudaError_t launch_pass_wide(int mode, int log_l, int log_c, const PassArgs& a, 
 
 // ---- column transforms ----------------------------------------------------------------------------
 
-// Tile width (log2 columns) of a column-transform pass, -1: none.
+// Tile width (log2 columns) of a column-transform pass, -1: none. First passes of 2^8 .. 2^10 values stay
+// with k_pass_tma, whose regrouped tiles are faster at the full clock (B200, 2^27 values, one pass of
+// 2^10 418 us against 453, 2^9 401 against 437) and level at the power-limited one (498 / 492, 473 / 476).
+// The others, wide against k_pass_tma's, power-limited: one pass of 2^11 572 -> 513 us, 2^12 619 -> 563
+// (555 -> 494 at the full clock), two passes with a wide second one 2^18 930 -> 885, 2^20 1008 -> 914 (863 ->
+// 822). Last passes of 2^8 and 2^9 values take tiles of 32 and 16 columns, which leave SMs idle on
+// small matrices: from 2^25 values on.
 static constexpr int column_wide_log_c(int mode, int log_l) {
-    return log_l == 12 ? (mode == 0 ? 1 : 2) : log_l == 11 ? (mode == 0 ? 2 : 3) : log_l == 10 ? (mode == 0 ? 3 : 4)
-           : log_l == 9 ? 4 : log_l == 8 ? 5 : -1;
+    return log_l == 12 ? (mode == 0 ? 1 : 2) : log_l == 11 ? (mode == 0 ? 2 : 3) : mode == 0 ? -1
+           : log_l == 10 ? 4 : log_l == 9 ? 4 : log_l == 8 ? 5 : -1;
 }
 
-// Measured against k_pass_tma's column passes (B200, warm): 2^27 values, one pass of 2^8 .. 2^12 values
-// 456 -> 438, 484 -> 471, 520 -> 488, 572 -> 513, 619 -> 563 us; two passes 2^16 859 -> 785, 2^17
-// 956 -> 889, 2^18 933 -> 860, 2^19 1028 -> 942, 2^20 1001 -> 891 us; 2^24 values 66 -> 65 (2^10), 75 -> 69
-// (2^11), 82 -> 76 us (2^12). Columns of 2^8 and 2^9 values take tiles of 32 and 16 columns, which
-// leave SMs idle on small matrices (2^20 values 5.1 -> 5.9 us, 2^24 114 -> 116): from 2^25 values on.
 bool pass_columns_wide_supported(int mode, int log_l, const PassArgs& a) {
     const int c = column_wide_log_c(mode, log_l);
     return c >= 0 && (log_l >= 10 || a.log2n >= 25) && a.log2n >= log_l + c && (mode == 0 || a.log_s >= c) &&
@@ -323,18 +324,17 @@ bool pass_columns_wide_supported(int mode, int log_l, const PassArgs& a) {
 }
 
 cudaError_t launch_pass_columns_wide(int mode, int log_l, const PassArgs& a, cudaStream_t stream) {
-#define OFB_WIDE_COLUMNS(LL) \
-    case LL: return mode == 0 ? launch_wide_w<LL, column_wide_log_c(0, LL), 0, false, false, true>(a, 1, stream) \
-                              : launch_wide_w<LL, column_wide_log_c(2, LL), 2, false, false, true>(a, 1, stream);
-    switch (log_l) {
-        OFB_WIDE_COLUMNS(12)
-        OFB_WIDE_COLUMNS(11)
-        OFB_WIDE_COLUMNS(10)
-        OFB_WIDE_COLUMNS(9)
-        OFB_WIDE_COLUMNS(8)
-    default: return cudaErrorInvalidValue;
-    }
+#define OFB_WIDE_COLUMNS(LL, M) \
+    if (log_l == LL && mode == M) return launch_wide_w<LL, column_wide_log_c(M, LL), M, false, false, true>(a, 1, stream);
+    OFB_WIDE_COLUMNS(12, 0)
+    OFB_WIDE_COLUMNS(11, 0)
+    OFB_WIDE_COLUMNS(12, 2)
+    OFB_WIDE_COLUMNS(11, 2)
+    OFB_WIDE_COLUMNS(10, 2)
+    OFB_WIDE_COLUMNS(9, 2)
+    OFB_WIDE_COLUMNS(8, 2)
 #undef OFB_WIDE_COLUMNS
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace ofb

@@ -76,3 +76,33 @@ def test_uneven_launches_back_to_back(ofb, count, lo, hi):
     # 2^16-point transforms grow by up to 2^16 per call pair: compare the bits, whatever they are
     assert torch.equal(out[0][0].view(torch.int32), out[1][0].view(torch.int32))
     assert torch.equal(out[0][1].view(torch.int32), out[1][1].view(torch.int32))
+
+
+def test_stream_capture_replays(ofb):
+    """Two chained calls of each kind recorded in one graph (dependent launches become programmatic
+    edges) give, replayed, the bits of the same calls outside it."""
+    import torch
+    calls = []
+    for log2n, batch in ((6, 300), (12, 1200), (13, 400), (14, 5), (15, 2), (15, 400), (18, 3), (20, 1), (24, 1)):
+        n = 1 << log2n
+        plan = ofb.Plan(n)
+        calls.append((2 * n * batch, lambda a, b, s, p=plan, k=batch: p.dev_forward(a, b, k, s), plan))
+    c = ofb.Columns(1 << 13, 1 << 8)
+    calls.append((2 << 21, lambda a, b, s, c=c: c.execute(a, b, 0, s), c))
+    for floats, call, _keep in calls:
+        x = torch.randn(floats, device="cuda")
+        y, z, y2, z2 = (torch.zeros_like(x) for _ in range(4))
+        s = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        call(x.data_ptr(), y.data_ptr(), s.cuda_stream)
+        call(y.data_ptr(), z.data_ptr(), s.cuda_stream)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            call(x.data_ptr(), y2.data_ptr(), s.cuda_stream)
+            call(y2.data_ptr(), z2.data_ptr(), s.cuda_stream)
+        graph.replay()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, y2) and torch.equal(z, z2)
+        del graph
