@@ -1253,6 +1253,8 @@ static onefft_uneven *uneven_create(const onefft_desc *desc, size_t count, const
     u->args.counter = (int *)(base + desc_bytes + item_bytes + unit_bytes);
     u->args.done = (unsigned *)(u->args.counter + 1);
     u->args.nitems = (int)items.size();
+    u->args.nbig = 0;
+    while (u->args.nbig < (int)items.size() && items[u->args.nbig].log2n >= 13) ++u->args.nbig;
     u->args.left = u->args.done + items.size() + 1;
     if (e == cudaSuccess) e = cudaMemset(u->args.counter, 0, ctr_bytes);
     if (e == cudaSuccess) e = cudaMemcpy(base, sorted.data(), count * sizeof(onefft_desc), cudaMemcpyHostToDevice);

@@ -324,8 +324,9 @@ __global__ void __launch_bounds__(kUnevenThreads, 4) k_uneven(UnevenArgs a) {
         }
         __syncthreads();
         if (s_item) {
-            for (int k = tid; k <= a.nitems; k += kUnevenThreads) a.done[k] = 0;
-            if (tid == 0) *a.counter = 0, *a.left = 0;
+            // only transforms of 2^13 .. 2^16, which come first, count steps; then the abort word
+            for (int k = tid; k < a.nbig; k += kUnevenThreads) a.done[k] = 0;
+            if (tid == 0) a.done[a.nitems] = 0, *a.counter = 0, *a.left = 0;
         }
     }
 }

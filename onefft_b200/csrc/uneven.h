@@ -69,6 +69,7 @@ struct UnevenArgs {
     const UnevenUnit *units;
     int nunits;
     unsigned *done;
+    int nbig;        // items of 2^13 .. 2^16 (the first ones)
     unsigned *left;  // blocks that have left; the last one zeroes all counters again (NULL: the caller does)
     unsigned *err;  // set when a pass-1 unit's bounded wait for its pass 0 ran out
     const float2 *stw[kUnevenMaxLog2 + 1][2];  // stage tables: [m][0] single kernel / pass 0, [m][1] pass 1
