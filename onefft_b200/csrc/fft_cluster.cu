@@ -21,13 +21,13 @@ cudaError_t set_expire_waits_cluster(int on) {
 //  - Block s transforms its rows (B values each) two adjacent rows a thread, and stores 16-byte pairs:
 //    512 contiguous bytes a warp.
 // The next transform's copy is issued when a block has read its rows, half a transform ahead.
-// Two cluster barriers a transform: one says that every landing buffer is free (arrived at early,
-// without a release, which would wait for the previous transform's stores: 2000 transforms 324 -> 292
-// us; waited for late), one that the rows have arrived. A block's columns are the same for every
+// Two cluster barriers a transform: one says that every landing buffer is free (arrived at early, waited
+// for late), one that the rows have arrived. The first arrival releases this thread's reads of its
+// landing buffer to the peers that overwrite it, and nothing else (cluster_arrive_shared). A block's columns are the same for every
 // transform it takes, so the inter-pass factors are computed once per launch.
 //
-// Measured on a B200, warm, against the two passes: 2000 x 2^15 292 us against 367, 512 x 2^15 86
-// against 100 (two trips of 268 MB through HBM at the board's power limit). What bounds it: a block's
+// Measured on a B200, warm, against the two passes: 2000 x 2^15 293 us against 331, 512 x 2^15 86
+// against 93 (two trips of 268 MB through HBM at the board's power limit). What bounds it: a block's
 // load, two transforms and exchanges follow each other (one block an SM, 10.4 us a transform), so it needs
 // many transforms per cluster: 160 x 2^15 (three rounds of 72 clusters) 40 us against 29. The same
 // with four blocks for 2^16 was slower than two passes (1000 transforms 405 us against 372; 33 clusters
@@ -47,8 +47,13 @@ struct Cluster {
 };
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-// Without the release's wait for this thread's own writes to memory (the previous transform's output).
-__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+// The same for this thread's accesses to its own block's shared memory only: a relaxed arrival orders
+// nothing by itself, so the fence before it does, without the full release's wait for this thread's
+// writes to global memory (the previous transform's output: 2000 transforms 293 us with the fence, 324 with a full release).
+__device__ __forceinline__ void cluster_arrive_shared() {
+    asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ unsigned cluster_map(unsigned addr, unsigned rank) {
     unsigned r;
@@ -122,7 +127,7 @@ __global__ void __cluster_dims__(Q, 1, 1) __launch_bounds__(512, 1)
                 asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_map(smem_u32(failed), s)), "r"(1u) : "memory");
             asm volatile("fence.acq_rel.cluster;" ::: "memory");
         }
-        cluster_arrive_relaxed();  // this landing buffer is free: its reads ended at the block barrier above
+        cluster_arrive_shared();  // this thread's reads of the landing buffer are done
         pair_stage<8, 0>(v, j, a.stw);
         {
             float2* w = ex + 16 * j * 32 + p;

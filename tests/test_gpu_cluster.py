@@ -59,3 +59,21 @@ def test_expired_wait_is_reported(ofb):
     want = torch.fft.fft(torch.view_as_complex(x.view(-1, 2)).view(batch, N)[-1].to(torch.complex128))
     got = torch.view_as_complex(out.view(-1, 2)).view(batch, N)[-1]
     assert float((got - want).abs().norm() / want.abs().norm()) < 1e-6
+
+
+def test_many_rounds_forward(ofb):
+    """Forward without weights, where nothing but the cluster's barriers stands between a block's reads
+    of its landing buffer and the peer's stores into it: about 70 transforms a cluster, several launches
+    in a row, every one with the passes' bits."""
+    import torch
+    batch = 5000
+    x = torch.randn(2 * N * batch, device="cuda", generator=torch.Generator(device="cuda").manual_seed(5))
+    out, want = torch.empty_like(x), torch.empty_like(x)
+    default, passes = ofb.Plan(N), ofb.Plan(N, split=(8, 7), l2_keep=False)
+    passes.dev_forward(x.data_ptr(), want.data_ptr(), batch)
+    for _ in range(8):
+        out.fill_(7.0)
+        default.dev_forward(x.data_ptr(), out.data_ptr(), batch)
+        torch.cuda.synchronize()
+        default.check()
+        assert torch.equal(out, want)
