@@ -88,10 +88,7 @@ __global__ void __cluster_dims__(Q, 1, 1) __launch_bounds__(512, 1)
         load(t);
     }
     const float2 *pre = nullptr, *post = nullptr;
-    if constexpr (W) {
-        dependent_wait();  // every thread reads the caller's weights
-        pre = after_wait(a.pre), post = after_wait(a.post);
-    }
+    if constexpr (W) pre = a.pre, post = a.post;
     // first pass: loads and stage 0 as lane j of columns 2 p, 2 p + 1; stage 1 as lanes 2 u, 2 u + 1 of
     // column c
     const int p = tid & 31, j = tid >> 5, c = tid & 63, u = tid >> 6;
@@ -246,7 +243,7 @@ static cudaError_t launch_cluster_w(const PassArgs& a, const float2* stw_b, long
     if ((long long)clusters > batch) clusters = (int)batch;
     CUtensorMap tin;
     if (!make_map(&tin, a.in, 0, G::LOG_N, 8, 6, G::LOG_B, (int)batch)) return cudaErrorInvalidValue;
-    return launch_dependent(kernel, dim3((unsigned)(clusters * Q)), G::THREADS, G::SMEM, stream, a, stw_b, tin, batch);
+    return launch_kernel<!W>(kernel, dim3((unsigned)(clusters * Q)), G::THREADS, G::SMEM, stream, a, stw_b, tin, batch);
 }
 
 cudaError_t launch_cluster(const PassArgs& a, const float2* stw_b, int inverse, long long batch, cudaStream_t stream) {

@@ -32,13 +32,6 @@ __device__ __forceinline__ void dependent_launch() {
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 __device__ __forceinline__ void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// The same pointer, defined only here: read-only-path loads through it may be hoisted over the
-// block's barriers, but not above the dependent_wait() before it.
-template <class T>
-__device__ __forceinline__ const T* after_wait(const T* p) {
-    asm volatile("" : "+l"(p));
-    return p;
-}
 
 // ---- complex helpers ---------------------------------------------------------------------------
 

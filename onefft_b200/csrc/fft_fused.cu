@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(1 << (LOG_L + LOG_C - 4), LOG_L >= 11 ? 65536 
     const bool active = g < batch;
     float2 v[16];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) v[k] = active ? ld_stream(x + (g << LOG_L) + j + T * k) : make_float2(0.f, 0.f);
+    for (int k = 0; k < 16; ++k) v[k] = active ? ld_cached(x + (g << LOG_L) + j + T * k) : make_float2(0.f, 0.f);
     tile_fft<LOG_L, 1>(v, j, stw, smem, c << LOG_L);
     // v[k] = y[j + T k]: loss terms and the scaled spectrum 2 w^2 y
     float part = 0.f;

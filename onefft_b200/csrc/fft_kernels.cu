@@ -88,7 +88,6 @@ __global__ void __launch_bounds__(256) k_tiny(const float2* __restrict__ in, flo
     float2* dst = out + (first << LOG_N);
     dependent_launch();
     dependent_wait();
-    if constexpr (W) pre = after_wait(pre), post = after_wait(post);
     for (int i = threadIdx.x; i < total; i += 256) s[spad(i)] = ld_stream(src + i);
     __syncthreads();
 #pragma unroll
@@ -180,7 +179,8 @@ __device__ __forceinline__ void batched_tile_staged(const float2* __restrict__ i
 
 // INV: the direction as a compile-time constant (the re/im exchanges on load and store then
 // cost nothing in the forward kernel and no selects in the inverse one).
-template <int LOG_L, int LOG_C, bool W, int INV>
+// L1: loads cached there (ld_cached), in an ordinary launch.
+template <int LOG_L, int LOG_C, bool W, int INV, bool L1>
 __global__ void __launch_bounds__(1 << (LOG_L + LOG_C - 4))
     k_batched(const float2* __restrict__ in, float2* __restrict__ out, long long batch,
               const float2* __restrict__ stw, const float2* __restrict__ pre, const float2* __restrict__ post) {
@@ -188,12 +188,11 @@ __global__ void __launch_bounds__(1 << (LOG_L + LOG_C - 4))
     const int tid = threadIdx.x;
     dependent_launch();
     dependent_wait();
-    if constexpr (W) pre = after_wait(pre), post = after_wait(post);
     if constexpr (LOG_L <= 6) {
         batched_tile_staged<LOG_L, LOG_C, INV, W>(in, out, batch, stw, smem, tid, pre, post);
     } else {
         const long long g = ((long long)blockIdx.x << LOG_C) + (tid >> (LOG_L - 4));
-        batched_tile<LOG_L, LOG_C, false, W>(in + (g << LOG_L), out + (g << LOG_L), g < batch, INV, stw, smem, tid,
+        batched_tile<LOG_L, LOG_C, L1, 0, W>(in + (g << LOG_L), out + (g << LOG_L), g < batch, INV, stw, smem, tid,
                                              pre, post);
     }
 }
@@ -218,21 +217,21 @@ bool batched_log_c_supported(int log_l, int log_c) {
     return log_c == b || (log_c >= 0 && log_c >= b - 1 && log_c <= b + 1 && log_l + log_c <= 13);
 }
 
-template <int LOG_L, bool W, int LOG_C>
+template <int LOG_L, bool W, bool L1, int LOG_C>
 static cudaError_t launch_batched_w(const float2* in, float2* out, long long batch, const float2* stw, int inverse,
                                     cudaStream_t stream, const float2* pre, const float2* post) {
     constexpr int THREADS = 1 << (LOG_L + LOG_C - 4);
     constexpr int SMEM = smem_bytes(LOG_L, LOG_C);
-    auto kernel = inverse ? k_batched<LOG_L, LOG_C, W, 1> : k_batched<LOG_L, LOG_C, W, 0>;
+    auto kernel = inverse ? k_batched<LOG_L, LOG_C, W, 1, L1> : k_batched<LOG_L, LOG_C, W, 0, L1>;
     static std::atomic<unsigned long long> done_fwd{0}, done_inv{0};
-    cudaError_t attr = inverse ? smem_limit((const void*)k_batched<LOG_L, LOG_C, W, 1>, SMEM, done_inv)
-                               : smem_limit((const void*)k_batched<LOG_L, LOG_C, W, 0>, SMEM, done_fwd);
+    cudaError_t attr = inverse ? smem_limit((const void*)k_batched<LOG_L, LOG_C, W, 1, L1>, SMEM, done_inv)
+                               : smem_limit((const void*)k_batched<LOG_L, LOG_C, W, 0, L1>, SMEM, done_fwd);
     if (attr != cudaSuccess) return attr;
     const long long per_block = 1ll << LOG_C;
     long long blocks = (batch + per_block - 1) / per_block;
     while (blocks > 0) {  // gridDim.x limit 2^31-1
         long long now = blocks < 0x7fffffffll ? blocks : 0x7fffffffll;
-        const cudaError_t e = launch_dependent(kernel, dim3((unsigned)now), THREADS, SMEM, stream, in, out, batch, stw, pre, post);
+        const cudaError_t e = launch_kernel<!L1>(kernel, dim3((unsigned)now), THREADS, SMEM, stream, in, out, batch, stw, pre, post);
         if (e != cudaSuccess) return e;
         long long done = now * per_block;
         in += done << LOG_L;
@@ -243,24 +242,36 @@ static cudaError_t launch_batched_w(const float2* in, float2* out, long long bat
     return cudaGetLastError();
 }
 
-template <int LOG_L, bool W>
+template <int LOG_L, bool W, bool L1>
 static cudaError_t launch_batched_c(const float2* in, float2* out, long long batch, const float2* stw, int inverse,
                                     cudaStream_t stream, const float2* pre, const float2* post, int log_c) {
     constexpr int B = default_batched_log_c(LOG_L);
     if constexpr (B >= 1)
         if (log_c == B - 1)
-            return launch_batched_w<LOG_L, W, B - 1>(in, out, batch, stw, inverse, stream, pre, post);
+            return launch_batched_w<LOG_L, W, L1, B - 1>(in, out, batch, stw, inverse, stream, pre, post);
     if constexpr (LOG_L + B + 1 <= 13)
         if (log_c == B + 1)
-            return launch_batched_w<LOG_L, W, B + 1>(in, out, batch, stw, inverse, stream, pre, post);
-    return launch_batched_w<LOG_L, W, B>(in, out, batch, stw, inverse, stream, pre, post);
+            return launch_batched_w<LOG_L, W, L1, B + 1>(in, out, batch, stw, inverse, stream, pre, post);
+    return launch_batched_w<LOG_L, W, L1, B>(in, out, batch, stw, inverse, stream, pre, post);
 }
+
+// A warp of the direct tiles reads pieces of 64 bytes at n = 2^7 and of 128 at 2^8. Large batches in whose
+// reads such a piece is less than a line, or straddles its sectors, run as ordinary launches with loads
+// cached in L1. Measured on a B200, cached and ordinary / through L2 and dependent, us: 2^7 aligned 2^22
+// values 12.4 / 9.7, 2^23 24.8 / 24.4, 2^24 46.5 / 47.6, 2^26 173 / 181; off the sector boundary 12.4 /
+// 11.2, 26.8 / 28.5, 49.5 / 54.2, 185 / 208; 2^8 aligned 2^24 45.1 / 43.1, 2^26 163 / 159; off the boundary
+// 2^22 12.4 / 9.9, 2^23 25.2 / 25.4, 2^24 46.3 / 47.9, 2^26 170 / 182.
+constexpr long long kCachedValues = 3 << 21;
 
 template <int LOG_L>
 static cudaError_t launch_batched_t(const float2* in, float2* out, long long batch, const float2* stw, int inverse,
                                     cudaStream_t stream, const float2* pre, const float2* post, int log_c) {
-    if (pre || post) return launch_batched_c<LOG_L, true>(in, out, batch, stw, inverse, stream, pre, post, log_c);
-    return launch_batched_c<LOG_L, false>(in, out, batch, stw, inverse, stream, nullptr, nullptr, log_c);
+    if (pre || post) return launch_batched_c<LOG_L, true, true>(in, out, batch, stw, inverse, stream, pre, post, log_c);
+    if constexpr (LOG_L == 7 || LOG_L == 8) {
+        if ((batch << LOG_L) >= kCachedValues && (LOG_L == 7 || ((uintptr_t)in & 31)))
+            return launch_batched_c<LOG_L, false, true>(in, out, batch, stw, inverse, stream, nullptr, nullptr, log_c);
+    }
+    return launch_batched_c<LOG_L, false, false>(in, out, batch, stw, inverse, stream, nullptr, nullptr, log_c);
 }
 
 template <int LOG_N>
@@ -271,8 +282,9 @@ static cudaError_t launch_tiny_t(const float2* in, float2* out, long long batch,
     long long blocks = (batch + PB - 1) / PB;
     while (blocks > 0) {
         long long now = blocks < 0x7fffffffll ? blocks : 0x7fffffffll;
-        const cudaError_t e = launch_dependent(w ? k_tiny<LOG_N, true> : k_tiny<LOG_N, false>, dim3((unsigned)now), 256, 0,
-                                               stream, in, out, batch, inverse, pre, post);
+        const cudaError_t e =
+            w ? launch_kernel<false>(k_tiny<LOG_N, true>, dim3((unsigned)now), 256, 0, stream, in, out, batch, inverse, pre, post)
+              : launch_kernel<true>(k_tiny<LOG_N, false>, dim3((unsigned)now), 256, 0, stream, in, out, batch, inverse, pre, post);
         if (e != cudaSuccess) return e;
         long long done = now * PB;
         in += done << LOG_N;
@@ -337,7 +349,7 @@ static cudaError_t launch_pass_w(const PassArgs& a, int batch, cudaStream_t stre
     while (batch > 0) {
         int now = batch < 65535 ? batch : 65535;
         grid.y = (unsigned)now;
-        const cudaError_t e = launch_dependent(kernel, grid, THREADS, SMEM, stream, b);
+        const cudaError_t e = launch_kernel<!W>(kernel, grid, THREADS, SMEM, stream, b);
         if (e != cudaSuccess) return e;
         b.in += (long long)now << a.log2n;
         b.out += (long long)now << a.log2n;
@@ -409,7 +421,7 @@ static cudaError_t launch_columns_t(const PassArgs& a, cudaStream_t stream) {
     if (a.log2n > 31 || a.log2n < LOG_L + LOG_C) return cudaErrorInvalidValue;
     PassArgs b = a;
     b.tli = 31;
-    return launch_dependent(kernel, dim3(1u << (a.log2n - LOG_L - LOG_C)), THREADS, SMEM, stream, b);
+    return launch_kernel<true>(kernel, dim3(1u << (a.log2n - LOG_L - LOG_C)), THREADS, SMEM, stream, b);
 }
 
 cudaError_t launch_pass_columns(int mode, int log_l, const PassArgs& a, cudaStream_t stream) {

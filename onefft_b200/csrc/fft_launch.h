@@ -30,9 +30,11 @@ inline cudaError_t smem_limit(const void* kernel, int bytes, std::atomic<unsigne
 // kernel's prologue take (1-3 us) then no longer lies between two kernels of a stream. Measured on a
 // B200, calls back to back: one 2^20 transform (two kernels) 16.4 -> 12.7 us, 2^17 10.3 -> 6.1 us,
 // 2^22 41.8 -> 35.1 us, 2^24 139 -> 132 us, 16 x 2^15 12.3 -> 7.1 us, 100003 x 64 20.9 -> 18.5 us.
-template <class... P, class... A>
-inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
-                                    const A&... args) {
+// DEPENDENT = false: an ordinary launch, for kernels that read the caller's weights through the
+// read-only path (ld_stream, fft_tiles.cuh); they may still release their successor early.
+template <bool DEPENDENT, class... P, class... A>
+inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
+                                 const A&... args) {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -42,7 +44,7 @@ inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, unsigned th
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = DEPENDENT ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 

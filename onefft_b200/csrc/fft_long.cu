@@ -120,10 +120,6 @@ __global__ void __launch_bounds__(256, B == 2 ? 2 : 1)
         mbar_expect_tx(bar, BYTES);
         bulk_load(long_smem, in + (b << LOG_N), BYTES, bar);
     }
-    if constexpr (W) {
-        dependent_wait();  // every thread reads the caller's weights
-        pre = after_wait(pre), post = after_wait(post);
-    }
     __syncthreads();  // the barrier is initialised before anyone waits on it
     for (; b < batch; b += gridDim.x, parity ^= 1u) {
         const bool ok = !g_expire_waits && mbar_wait(bar, parity);
@@ -206,7 +202,7 @@ static cudaError_t launch_long_w(const float2* in, float2* out, long long batch,
         grid_of[dev & 63].store(grid, std::memory_order_relaxed);
     }
     if ((long long)grid > batch) grid = (int)batch;
-    return launch_dependent(kernel, dim3((unsigned)grid), G::THREADS, G::SMEM, stream, in, out, batch, stw, err, pre, post);
+    return launch_kernel<!W>(kernel, dim3((unsigned)grid), G::THREADS, G::SMEM, stream, in, out, batch, stw, err, pre, post);
 }
 
 template <int B>

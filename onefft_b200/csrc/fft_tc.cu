@@ -12,7 +12,7 @@ __global__ void __launch_bounds__(1 << (LOG_L + LOG_C - 4))
     extern __shared__ float2 smem[];
     const int tid = threadIdx.x;
     const long long g = ((long long)blockIdx.x << LOG_C) + (tid >> (LOG_L - 4));
-    batched_tile<LOG_L, LOG_C, TERMS>(in + (g << LOG_L), out + (g << LOG_L), g < batch, inverse, stw, smem, tid);
+    batched_tile<LOG_L, LOG_C, true, TERMS>(in + (g << LOG_L), out + (g << LOG_L), g < batch, inverse, stw, smem, tid);
 }
 
 template <int LOG_L, int LOG_C, int MODE, int TERMS>

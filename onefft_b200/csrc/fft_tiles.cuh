@@ -97,19 +97,26 @@ __device__ __forceinline__ long long column_dst(const PassArgs& a, unsigned long
     return (long long)(((((k >> a.xlog_blk) << a.xlog_cols) + b) << a.xlog_blk) + (k & ((1ull << a.xlog_blk) - 1)));
 }
 
-// Loads of the caller's buffers. They are volatile and coherent, not read-only-path loads, so that
-// none moves above the dependent_wait() that orders it after the previous kernel's writes. Data that
-// the kernel itself overwrites (the in-place passes) is loaded through L2 only: blocks of one pass
-// may share a 32-byte sector, and the next kernel, started early on the same SM, could find the copy
-// that a block of this one left in L1 before its neighbour wrote the sector.
+// Loads of the caller's data, through L2 only. The next kernel of the stream may be resident on this SM
+// already (dependent_launch) and reads its input once dependent_wait() has returned; if a block of this
+// kernel, or of one before it, had left a copy of that 32-byte sector in this SM's L1 before another SM
+// wrote the sector, the read could find the copy. That takes a kernel that reads and writes one
+// sector: the in-place passes on buffers that are only 8-byte aligned, an input that ends or begins
+// in the sector where the output begins or ends. Whether the wait alone discards such copies is not
+// established here; with no such data in L1 it does not matter. Volatile: none moves above the wait.
+// ld_cached is for kernels whose SMs hold no older copy: ordinary launches, and the uneven kernel, which
+// fences after its wait. They gain from L1 where a warp reads pieces shorter than a line.
+// Pointwise weights are read by every block and belong in L1 (through L2 only, a batch of 2^24 values in
+// transforms of 4 took 234 us instead of 52, in transforms of 2^14 154 instead of 94): they are __ldg
+// loads, and kernels that read them are launched as ordinary successors (launch_kernel<false>).
 __device__ __forceinline__ float2 ld_stream(const float2* p) {
     float2 v;
-    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
     return v;
 }
-__device__ __forceinline__ float2 ld_l2(const float2* p) {
+__device__ __forceinline__ float2 ld_cached(const float2* p) {
     float2 v;
-    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
     return v;
 }
 // The array between passes may be kept in L2 for the next pass (evict last).
@@ -175,7 +182,7 @@ __device__ __forceinline__ void tiny_transform(const float2* __restrict__ src, f
     float2 a[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-        a[i] = __ldg(src + i);
+        a[i] = ld_cached(src + i);
         if constexpr (W) {
             if (pre) a[i] = cmul(a[i], __ldg(pre + i));
         }
@@ -198,8 +205,8 @@ __device__ __forceinline__ void tiny_transform(const float2* __restrict__ src, f
 // c = tid / (L/16) and butterfly lane j = tid mod (L/16). src / dst point at this thread's
 // transform; inactive columns (past the end of a batch) compute on zeros and store nothing.
 // TC: 0 = FP32 stages; 3 or 6 = the split-BF16 tensor-core stages with that many product terms
-// (fft_tc.cuh). W, pre, post as tiny_transform.
-template <int LOG_L, int LOG_C, int TC = 0, bool W = false>
+// (fft_tc.cuh). W, pre, post as tiny_transform. L1: the loads may be cached there (ld_cached).
+template <int LOG_L, int LOG_C, bool L1, int TC = 0, bool W = false>
 __device__ __forceinline__ void batched_tile(const float2* __restrict__ src, float2* __restrict__ dst, bool active,
                                              int inverse, const float2* __restrict__ stw, float2* smem, int tid,
                                              const float2* __restrict__ pre = nullptr,
@@ -211,7 +218,8 @@ __device__ __forceinline__ void batched_tile(const float2* __restrict__ src, flo
     dst += j;
     float2 v[16];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) v[k] = active ? ld_stream(src + T * k) : make_float2(0.f, 0.f);
+    for (int k = 0; k < 16; ++k) 
+        v[k] = !active ? make_float2(0.f, 0.f) : L1 ? ld_cached(src + T * k) : ld_stream(src + T * k);
     if constexpr (W) {  // after all loads: a test of `pre` between them would keep them apart
         if (pre) {
 #pragma unroll
@@ -243,7 +251,7 @@ __device__ __forceinline__ void batched_tile(const float2* __restrict__ src, flo
 // over the 2^LOG_C L / 16 threads of the tile.
 // W: the first pass multiplies its input by a.pre, the last pass its output by a.post (see
 // PassArgs); without W they are not compiled in.
-// CG: later passes load through L2 only (ld_l2), for data that other blocks may have written while
+// CG: later passes load through L2 only (ld_stream), for data that other blocks may have written while
 // this SM's L1 holds an older copy.
 // X: a pass of a column transform (PassArgs' column fields): MODE 0 takes its inter-pass factor
 // from the column fields and, with colstore, writes the column layout (and a.swap_out: it is
@@ -286,9 +294,9 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, unsigned t, long lo
         pass_twiddle_rows<LOG_L, LOG_C, MODE>(a, col0, tws, tid, C * T);
         wjf = pass_twiddle_lane<LOG_L>(a, MODE == 0 ? col0 + cl : (col0 >> a.log_s) << a.log_s, jl);
     }
-    dependent_wait();  // (returns at once in the uneven kernel, whose launches are not dependent ones)
+    dependent_wait();  // (the uneven kernel has waited already)
     const float2 *pre = nullptr, *post = nullptr;
-    if constexpr (W) pre = after_wait(a.pre), post = after_wait(a.post);
+    if constexpr (W) pre = a.pre, post = a.post;
     // element j + T k of the column: p0 + k * estep
     const long long estep = (long long)T << a.log_s;
     const long long off0 = toff + base + ((long long)j << a.log_s);
@@ -298,7 +306,7 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, unsigned t, long lo
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
             // The first pass streams the input; later passes read and write `out` in place.
-            float2 x = MODE == 0 ? ld_stream(p0 + k * estep) : CG ? ld_l2(p0 + k * estep) : p0[k * estep];
+            float2 x = MODE == 0 || CG ? ld_stream(p0 + k * estep) : p0[k * estep];
             if constexpr (W && MODE == 0) {
                 if (pre) x = cmul(x, __ldg(pre + (off0 - toff) + k * estep));
             }

@@ -136,10 +136,7 @@ __device__ __forceinline__ bool tma_tile(const PassArgs& a, const CUtensorMap* t
         return false;
     }
     const float2 *pre = nullptr, *post = nullptr;
-    if constexpr (W) {
-        dependent_wait();  // this thread reads the caller's weights itself
-        pre = after_wait(a.pre), post = after_wait(a.post);
-    }
+    if constexpr (W) pre = a.pre, post = a.post;
     landed();
     float2 v[16];
 #pragma unroll
@@ -454,7 +451,7 @@ static cudaError_t launch_tma_w(const PassArgs& a, int batch, cudaStream_t strea
     dim3 grid(a.ntiles ? a.ntiles : 1u << (a.log2n - LOG_L - LOG_C), (unsigned)batch, 1);
     PassArgs b = a;
     if (!a.ntiles) b.tli = 31;
-    return launch_dependent(kernel, grid, THREADS, SMEM, stream, b, tin, tout);
+    return launch_kernel<!W>(kernel, grid, THREADS, SMEM, stream, b, tin, tout);
 }
 
 // Tile shapes with a TMA kernel (the only ones pass_tma_supported accepts): widths 2 .. 16
@@ -546,7 +543,7 @@ static cudaError_t launch_columns_tma_t(const PassArgs& a, cudaStream_t stream) 
     if (!make_map(&tin, a.in, MODE, a.log2n, LOG_L, LOG_C, a.log_s, 1)) return cudaErrorInvalidValue;
     PassArgs b = a;
     b.tli = 31;
-    return launch_dependent(kernel, dim3(1u << (a.log2n - LOG_L - LOG_C)), THREADS, SMEM, stream, b, tin, tin);
+    return launch_kernel<true>(kernel, dim3(1u << (a.log2n - LOG_L - LOG_C)), THREADS, SMEM, stream, b, tin, tin);
 }
 
 cudaError_t launch_pass_columns_tma(int mode, int log_l, const PassArgs& a, cudaStream_t stream) {

@@ -135,10 +135,7 @@ __global__ void __launch_bounds__(Wide<LOG_L, LOG_C>::THREADS, LOG_L + LOG_C >= 
         load(t);
     }
     const float2 *pre = nullptr, *post = nullptr;
-    if constexpr (W) {
-        dependent_wait();  // every thread reads the caller's weights
-        pre = after_wait(a.pre), post = after_wait(a.post);
-    }
+    if constexpr (W) pre = a.pre, post = a.post;
     __syncthreads();  // the barrier is initialised before anyone waits on it
     for (; t < tiles; t += gridDim.x, parity ^= 1u) {
         const unsigned col0 = (t & ((1u << log_tiles) - 1)) << LOG_C;
@@ -267,7 +264,7 @@ static cudaError_t launch_wide_w(const PassArgs& a, int batch, cudaStream_t stre
     const int log_tiles = a.log2n - LOG_L - LOG_C;
     const unsigned tiles = (unsigned)batch << log_tiles;
     if ((unsigned)grid > tiles) grid = (int)tiles;
-    return launch_dependent(kernel, dim3((unsigned)grid), G::THREADS, G::SMEM, stream, a, tin, tiles, log_tiles);
+    return launch_kernel<!W>(kernel, dim3((unsigned)grid), G::THREADS, G::SMEM, stream, a, tin, tiles, log_tiles);
 }
 
 template <int LOG_L, int LOG_C, int MODE>

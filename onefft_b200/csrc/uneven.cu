@@ -241,7 +241,7 @@ __device__ __forceinline__ void batch_item(const UnevenArgs& a, const UnevenItem
     const int c = tid >> (M - 4);
     const bool active = c < w.count;
     const onefft_desc d = a.desc[w.first + (active ? c : 0)];
-    batched_tile<M, LOG_C>(a.in + d.offset, a.out + d.offset, active, d.inverse, a.stw[M][0], smem, tid);
+    batched_tile<M, LOG_C, true>(a.in + d.offset, a.out + d.offset, active, d.inverse, a.stw[M][0], smem, tid);
 }
 
 template <int M>
@@ -264,7 +264,10 @@ __global__ void __launch_bounds__(kUnevenThreads, 4) k_uneven(UnevenArgs a) {
     const int tid = threadIdx.x;
     const int count = a.units ? a.nunits : a.nitems;
     dependent_wait();
-    if (tid == 0) s_item = atomicAdd(a.counter, 1);
+    if (tid == 0) {
+        __threadfence();  // the block's loads may go through L1 (ld_cached): nothing older stays there
+        s_item = atomicAdd(a.counter, 1);
+    }
     __syncthreads();
     int s = s_item;
     for (;; s = s_item) {
