@@ -176,7 +176,7 @@ cudaError_t setup(NoAllocDevice &d, int device, cudaStream_t stream) {
     d.args.desc = d.desc;
     d.args.items = d.items;
     d.args.counter = d.counter;
-    d.kernel = uneven_kernel(d.args.split);  // the tuned kernel, as onefft_uneven_create
+    d.kernel = uneven_kernel(d.args.split, true);  // the tuned kernel, as onefft_uneven_create
     d.smem = uneven_smem_bytes();
     if (d.smem > 48 * 1024 &&
         (e = cudaFuncSetAttribute(d.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem)) != cudaSuccess)

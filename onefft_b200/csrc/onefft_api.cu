@@ -1065,6 +1065,7 @@ struct onefft_uneven {
     void *mem;  // sorted descriptors, work items, units, queue counter + per-item step counters
     unsigned *err_host;  // error word (mapped pinned host memory), as the plans'
     UnevenArgs args;
+    const void *kernel;
     int grid;
     int smem;
     cudaGraph_t graph;
@@ -1245,6 +1246,7 @@ static onefft_uneven *uneven_create(const onefft_desc *desc, size_t count, const
     } else {
         u->err_host = nullptr;
     }
+    u->kernel = uneven_kernel(u->args.split, items[0].log2n >= 13);  // the largest come first
     char *base = (char *)u->mem;
     u->args.desc = (const onefft_desc *)base;
     u->args.items = (const UnevenItem *)(base + desc_bytes);
@@ -1267,8 +1269,8 @@ static onefft_uneven *uneven_create(const onefft_desc *desc, size_t count, const
     u->smem = uneven_smem_bytes();
     int per_sm = 0, sms = 0;
     if (e == cudaSuccess && u->smem > 48 * 1024)
-        e = cudaFuncSetAttribute(uneven_kernel(u->args.split), cudaFuncAttributeMaxDynamicSharedMemorySize, u->smem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, uneven_kernel(u->args.split), 256, u->smem);
+        e = cudaFuncSetAttribute(u->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, u->smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, u->kernel, 256, u->smem);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     u->grid = std::max(1, std::min(per_sm * sms, (int)items.size()));
     // graph: the persistent launch (its last block leaves the counters zeroed for the next one)
@@ -1276,7 +1278,7 @@ static onefft_uneven *uneven_create(const onefft_desc *desc, size_t count, const
     if (e == cudaSuccess) {
         void *params[1] = {&u->args};
         cudaKernelNodeParams kp{};
-        kp.func = (void *)uneven_kernel(u->args.split);
+        kp.func = (void *)u->kernel;
         kp.gridDim = dim3((unsigned)u->grid);
         kp.blockDim = dim3(256);
         kp.sharedMemBytes = (unsigned)u->smem;
@@ -1323,7 +1325,7 @@ extern "C" int onefft_uneven_execute(onefft_uneven *u, const float *d_in, float 
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         g_launches.fetch_add(1);
-        e = cudaLaunchKernelExC(&cfg, uneven_kernel(u->args.split), params);
+        e = cudaLaunchKernelExC(&cfg, u->kernel, params);
         return e == cudaSuccess ? 0 : cuda_error(e, "uneven batch launch");
     }
     if (u->args.in != (const float2 *)d_in || u->args.out != (float2 *)d_out) {
@@ -1331,7 +1333,7 @@ extern "C" int onefft_uneven_execute(onefft_uneven *u, const float *d_in, float 
         u->args.out = (float2 *)d_out;
         void *params[1] = {&u->args};
         cudaKernelNodeParams kp{};
-        kp.func = (void *)uneven_kernel(u->args.split);
+        kp.func = (void *)u->kernel;
         kp.gridDim = dim3((unsigned)u->grid);
         kp.blockDim = dim3(256);
         kp.sharedMemBytes = (unsigned)u->smem;

@@ -186,15 +186,18 @@ __device__ __noinline__ void big_item_call(const BigItemArgs b, float2* smem, in
 }
 
 // One 2^M transform with split CHOICE, or, for CHOICE = kSplitAtRunTime, the split the batch
-// was created with (UnevenArgs::split).
+// was created with (UnevenArgs::split). kNoLarge: the batch has no transform of 2^13 .. 2^16.
 constexpr int kSplitAtRunTime = -1;
+constexpr int kNoLarge = -2;
 
 template <int M, int CHOICE>
 __device__ __forceinline__ void big_choice(const UnevenArgs& a, const onefft_desc& d, float2* smem, int tid) {
     constexpr int I = M - 13;
     const BigItemArgs b{a.in + d.offset, a.out + d.offset, a.tw_lo[M], a.tw_hi[M],
                         a.stw[M][0],     a.stw[M][1],      a.lo_bits[M], d.inverse};
-    if constexpr (CHOICE != kSplitAtRunTime) {
+    if constexpr (CHOICE == kNoLarge) {
+        return;
+    } else if constexpr (CHOICE != kSplitAtRunTime) {
         big_item<M, kUnevenSplits[I][CHOICE][0], kUnevenSplits[I][CHOICE][1]>(b, smem, tid);
     } else {
         static_assert(kUnevenSplitChoices == 3, "one branch per compiled split");
@@ -214,7 +217,9 @@ __device__ __forceinline__ void step_choice(const UnevenArgs& a, int it, const o
     const BigItemArgs b{a.in + d.offset, a.out + d.offset, a.tw_lo[M], a.tw_hi[M],
                         a.stw[M][0],     a.stw[M][1],      a.lo_bits[M], d.inverse};
     unsigned* abort = a.done + a.nitems;
-    if constexpr (CHOICE != kSplitAtRunTime) {
+    if constexpr (CHOICE == kNoLarge) {
+        return;
+    } else if constexpr (CHOICE != kSplitAtRunTime) {
         big_step<M, kUnevenSplits[I][CHOICE][0], kUnevenSplits[I][CHOICE][1]>(b, a.done + it, abort, a.err, step, smem,
                                                                              tid);
     } else {
@@ -252,11 +257,14 @@ __device__ __forceinline__ void tiny_item(const UnevenArgs& a, const UnevenItem&
     }
 }
 
-// Four resident blocks per SM (64 registers, a few spilled values): measured on a B200 with
+// Four resident blocks per SM (64 registers): measured on a B200 with
 // 20000 transforms of 2^4 .. 2^16, 1.21 ms at 2 blocks per SM (128 registers), 1.14 ms at 3
 // (80 registers), 1.12 ms at 4; items are latency-bound tile sequences, so more resident blocks
 // hide more of each block's waits.
-// C13 .. C16: the split of each size 2^13 .. 2^16 (an index into kUnevenSplits, or kSplitAtRunTime).
+// Batches without transforms of 2^13 .. 2^16 run a kernel without their steps: beside them the small
+// items were allocated worse (15370 transforms of 2^4 .. 2^12 60.2 us, without 55.4; 5 blocks per SM at 48
+// registers 69.7).
+// C13 .. C16: the split of each size 2^13 .. 2^16 (an index into kUnevenSplits, kSplitAtRunTime or kNoLarge).
 template <int C13, int C14, int C15, int C16>
 __global__ void __launch_bounds__(kUnevenThreads, 4) k_uneven(UnevenArgs a) {
     extern __shared__ float2 smem[];
@@ -283,7 +291,7 @@ __global__ void __launch_bounds__(kUnevenThreads, 4) k_uneven(UnevenArgs a) {
             step = u.step;
         }
         const UnevenItem w = a.items[it];
-        if (step >= 0) {
+        if (C13 != kNoLarge && step >= 0) {
             const onefft_desc d = a.desc[w.first];
             switch (w.log2n) {
             case 13: step_choice<13, C13>(a, it, d, step, smem, tid); break;
@@ -346,10 +354,11 @@ int uneven_smem_bytes() {
 
 // The compiled kernels: every split inlined for the plain path's splits (choice 0 everywhere)
 // and for the tuned choices, and one that reads the choices from its arguments (any other
-// combination; the autotuner times candidates with it).
+// combination; the autotuner times candidates with it); without large transforms, the one that has none.
 int uneven_tuned_split(int m) { return m >= 13 && m <= 16 ? kUnevenTunedSplit[m - 13] : 0; }
 
-const void *uneven_kernel(const int *split) {
+const void *uneven_kernel(const int *split, bool large) {
+    if (!large) return (const void *)k_uneven<kNoLarge, kNoLarge, kNoLarge, kNoLarge>;
     bool plain = true, tuned = true;
     for (int m = 13; m <= kUnevenMaxLog2; ++m) {
         const int c = split ? split[m] : 0;

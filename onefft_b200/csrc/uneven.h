@@ -85,8 +85,9 @@ int uneven_split(int m, int choice, int pass);
 // The autotuned split choice of size 2^m (0 outside 13 .. 16).
 int uneven_tuned_split(int m);
 // Dynamic shared memory of k_uneven, and the kernel that runs split choices split[13 .. 16]
-// (NULL: choice 0 everywhere), for graph nodes / launches / occupancy.
+// (NULL: choice 0 everywhere; large = false: no transform of 2^13 .. 2^16), for graph nodes / launches /
+// occupancy.
 int uneven_smem_bytes();
-const void *uneven_kernel(const int *split);
+const void *uneven_kernel(const int *split, bool large);
 
 }  // namespace ofb

@@ -200,3 +200,31 @@ def test_uneven_rejects_bad_arguments(ofb):
     for bad in (-1, 3):
         with pytest.raises(ValueError):
             ofb.UnevenBatch([14], [0], [0], split={14: bad})
+
+
+@pytest.mark.parametrize("hi,count", [(0, 3), (3, 300), (7, 900), (12, 400), (12, 3000)])
+def test_kernel_without_large_transforms(ofb, hi, count):
+    """A batch without transforms of 2^13 .. 2^16 runs a kernel of its own: the plain path's bits, and those
+    of the kernel that a single 2^13 more selects; below and beyond the line of the direct launch."""
+    import torch
+    r = np.random.RandomState(hi * 1000 + count)
+    m = r.randint(0, hi + 1, count)
+    inv = r.randint(0, 2, count)
+    gap = r.randint(0, 3, count)  # odd offsets
+    off = np.concatenate([[0], np.cumsum((1 << m) + gap)[:-1]])
+    batch = ofb.UnevenBatch(m, inv, off)
+    span = batch.span
+    more = ofb.UnevenBatch(np.append(m, 13), np.append(inv, 0), np.append(off, span))
+    x = torch.randn(2 * (span + (1 << 13)), device="cuda", generator=torch.Generator(device="cuda").manual_seed(count))
+    a, b, c = (torch.full_like(x, 7.0) for _ in range(3))
+    batch.execute(x.data_ptr(), a.data_ptr())
+    more.execute(x.data_ptr(), b.data_ptr())
+    plans = {k: ofb.Plan(1 << int(k)) for k in np.unique(m)}
+    for k, i, o in zip(m, inv, off):
+        f = plans[k].dev_inverse if i else plans[k].dev_forward
+        f(x.data_ptr() + 8 * int(o), c.data_ptr() + 8 * int(o), 1)
+    torch.cuda.synchronize()
+    assert batch.status() == 0 and more.status() == 0
+    assert torch.equal(a, c)  # values between and after the transforms untouched
+    assert torch.equal(a[:2 * span], b[:2 * span])
+    assert not bool((b[2 * span:] == 7.0).any())
