@@ -349,7 +349,7 @@ static cudaError_t launch_pass_w(const PassArgs& a, int batch, cudaStream_t stre
     while (batch > 0) {
         int now = batch < 65535 ? batch : 65535;
         grid.y = (unsigned)now;
-        const cudaError_t e = launch_kernel<!W>(kernel, grid, THREADS, SMEM, stream, b);
+        const cudaError_t e = launch_kernel<true>(kernel, grid, THREADS, SMEM, stream, b);
         if (e != cudaSuccess) return e;
         b.in += (long long)now << a.log2n;
         b.out += (long long)now << a.log2n;

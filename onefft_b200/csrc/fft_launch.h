@@ -148,6 +148,8 @@ cudaError_t launch_pass01_fused(int l0, int c0, int l1, int c1, const PassArgs& 
 cudaError_t launch_pass_tma(int mode, int log_l, int log_c, const PassArgs& a, int batch, cudaStream_t stream);
 // Wide-tile persistent passes (fft_wide.cu): same arithmetic, arguments and requirements as
 // launch_pass_tma (no chunks); the shapes the tuned table marks (onefft_api.cu, kWideTile)
+// (pass_wide_weights: whether the kernel applies the weights that this pass has to).
+bool pass_wide_weights(int mode, int log_l, const PassArgs& a);
 cudaError_t launch_pass_wide(int mode, int log_l, int log_c, const PassArgs& a, int batch, cudaStream_t stream);
 // A column-transform pass through its wide-tile kernel (as launch_pass_columns_tma; a.out 16-byte aligned)
 bool pass_columns_wide_supported(int mode, int log_l, const PassArgs& a);

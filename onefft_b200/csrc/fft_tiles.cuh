@@ -106,12 +106,18 @@ __device__ __forceinline__ long long column_dst(const PassArgs& a, unsigned long
 // established here; with no such data in L1 it does not matter. Volatile: none moves above the wait.
 // ld_cached is for kernels whose SMs hold no older copy: ordinary launches, and the uneven kernel, which
 // fences after its wait. They gain from L1 where a warp reads pieces shorter than a line.
-// Pointwise weights are read by every block and belong in L1 (through L2 only, a batch of 2^24 values in
-// transforms of 4 took 234 us instead of 52, in transforms of 2^14 154 instead of 94): they are __ldg
-// loads, and kernels that read them are launched as ordinary successors (launch_kernel<false>).
+// Pointwise weights of the one-kernel sizes are read by every block and belong in L1 (through L2 only, a
+// batch of 2^24 values in transforms of 4 took 234 us instead of 52, in transforms of 2^14 154 instead of
+// 94): they are __ldg loads, and those kernels are launched as ordinary successors (launch_kernel<false>).
+// A pass reads each weight once per transform: ld_stream.
 __device__ __forceinline__ float2 ld_stream(const float2* p) {
     float2 v;
     asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_stream4(const float2* p) {  // 16-byte aligned
+    float4 v;
+    asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
     return v;
 }
 __device__ __forceinline__ float2 ld_cached(const float2* p) {
@@ -250,7 +256,7 @@ __device__ __forceinline__ void batched_tile(const float2* __restrict__ src, flo
 // Tile t covers 2^LOG_C adjacent columns of the transform at element offset `toff`; tid runs
 // over the 2^LOG_C L / 16 threads of the tile.
 // W: the first pass multiplies its input by a.pre, the last pass its output by a.post (see
-// PassArgs); without W they are not compiled in.
+// PassArgs; the pointer the pass uses is not NULL); without W they are not compiled in.
 // CG: later passes load through L2 only (ld_stream), for data that other blocks may have written while
 // this SM's L1 holds an older copy.
 // X: a pass of a column transform (PassArgs' column fields): MODE 0 takes its inter-pass factor
@@ -295,21 +301,21 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, unsigned t, long lo
         wjf = pass_twiddle_lane<LOG_L>(a, MODE == 0 ? col0 + cl : (col0 >> a.log_s) << a.log_s, jl);
     }
     dependent_wait();  // (the uneven kernel has waited already)
-    const float2 *pre = nullptr, *post = nullptr;
-    if constexpr (W) pre = a.pre, post = a.post;
     // element j + T k of the column: p0 + k * estep
     const long long estep = (long long)T << a.log_s;
     const long long off0 = toff + base + ((long long)j << a.log_s);
     float2 v[16];
     {
         const float2* p0 = a.in + off0;
+        if constexpr (W && MODE == 0) {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] = ld_stream(a.pre + (off0 - toff) + k * estep);
+        }
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
             // The first pass streams the input; later passes read and write `out` in place.
             float2 x = MODE == 0 || CG ? ld_stream(p0 + k * estep) : p0[k * estep];
-            if constexpr (W && MODE == 0) {
-                if (pre) x = cmul(x, __ldg(pre + (off0 - toff) + k * estep));
-            }
+            if constexpr (W && MODE == 0) x = cmul(x, v[k]);
             v[k] = a.swap_in ? swap_ri(x) : x;
         }
     }
@@ -363,9 +369,7 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, unsigned t, long lo
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
             float2 x = a.swap_out ? swap_ri(v[k]) : v[k];
-            if constexpr (W && MODE == 2) {
-                if (post) x = cmul(x, __ldg(post + (off0 - toff) + k * estep));
-            }
+            if constexpr (W && MODE == 2) x = cmul(x, ld_stream(a.post + (off0 - toff) + k * estep));
             if (MODE == 1 && a.l2_keep) st_policy(p0 + k * estep, x, keep);
             else p0[k * estep] = x;
         }

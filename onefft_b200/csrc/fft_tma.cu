@@ -57,7 +57,7 @@ __host__ __device__ constexpr int tma_smem_bytes(int log_l, int log_c) {
 // the same in every thread, if the copy's bounded wait expired: the tile then recorded the
 // failure in the plan's error word, let the copy land and wrote nothing.
 // W: the first pass multiplies its input by a.pre, the last pass its output by a.post
-// (instantiated only for weighted calls).
+// (instantiated only for weighted calls, launched only where that pointer is not NULL).
 // Hooks, for the persistent fused kernel: thread 0 calls ready() before issuing the copy (false:
 // the tile is not run and tma_tile returns false), and issued() right after issuing it, so that
 // work which waits on memory overlaps the copy; every thread calls landed() once the copy has
@@ -125,6 +125,22 @@ __device__ __forceinline__ bool tma_tile(const PassArgs& a, const CUtensorMap* t
         pass_twiddle_rows<LOG_L, LOG_C, MODE>(a, col0, tws, tid, C * T);
         wjf = pass_twiddle_lane<LOG_L>(a, MODE == 0 ? col0 + cl : (col0 >> a.log_s) << a.log_s, jl);
     }
+    float2 v[16];
+    if constexpr (W) dependent_wait();  // this thread reads the caller's weights itself
+    if constexpr (W && MODE == 2 && LOG_L >= 11) {
+        // Output weights into L2 ahead of their use: one or two blocks of these long columns run on an SM, and
+        // little overlaps the loads. B200, warm, us: 2^23 92.5 -> 87.6, 2^24 201 -> 190, 2 x 2^24 391 -> 372, 2 x 2^22
+        // 89.6 -> 85.7, 2^22 43.4 -> 45.2; with short columns it costs (2^28 3.37 -> 3.82 ms).
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(a.post + (unsigned)(q0 + c) + ((unsigned)(j + T * k) << a.log_s) +
+                                                          ((unsigned)h << (a.log_s + LOG_L))));
+    }
+    if constexpr (W && MODE == 0) {  // the weights first, in the registers of the values they multiply:
+        // those of input element col0 + c + (j + T k) S of the transform
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = ld_stream(a.pre + col0 + c + ((unsigned)(j + T * k) << a.log_s));
+    }
     // the barrier is initialised (and armed) before anyone waits on it
     if (__syncthreads_or(!go)) return false;  // nothing was issued: nothing to wait for
     const bool ok = !g_expire_waits && mbar_wait(bar, parity);
@@ -135,17 +151,11 @@ __device__ __forceinline__ bool tma_tile(const PassArgs& a, const CUtensorMap* t
         }
         return false;
     }
-    const float2 *pre = nullptr, *post = nullptr;
-    if constexpr (W) pre = a.pre, post = a.post;
     landed();
-    float2 v[16];
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
         float2 x = smem[(j + T * k) * C + c];
-        // input element col0 + c + (j + T k) S of the transform (first pass only)
-        if constexpr (W && MODE == 0) {
-            if (pre) x = cmul(x, __ldg(pre + col0 + c + ((unsigned)(j + T * k) << a.log_s)));
-        }
+        if constexpr (W && MODE == 0) x = cmul(x, v[k]);
         v[k] = a.swap_in ? swap_ri(x) : x;
     }
     __syncthreads();  // the dense tile is consumed; the exchanges reuse its memory
@@ -191,9 +201,8 @@ __device__ __forceinline__ bool tma_tile(const PassArgs& a, const CUtensorMap* t
             float2 x = a.swap_out ? swap_ri(v[k]) : v[k];
             // output element q0 + c + (j + T k) S + h L S of the transform, natural order (last pass)
             if constexpr (W && MODE == 2) {
-                if (post)
-                    x = cmul(x, __ldg(post + (unsigned)(q0 + c) + ((unsigned)(j + T * k) << a.log_s) +
-                                     ((unsigned)h << (a.log_s + LOG_L))));
+                x = cmul(x, ld_stream(a.post + (unsigned)(q0 + c) + ((unsigned)(j + T * k) << a.log_s) +
+                                      ((unsigned)h << (a.log_s + LOG_L))));
             }
             smem[(j + T * k) * C + c] = x;
         }
@@ -451,7 +460,7 @@ static cudaError_t launch_tma_w(const PassArgs& a, int batch, cudaStream_t strea
     dim3 grid(a.ntiles ? a.ntiles : 1u << (a.log2n - LOG_L - LOG_C), (unsigned)batch, 1);
     PassArgs b = a;
     if (!a.ntiles) b.tli = 31;
-    return launch_kernel<!W>(kernel, grid, THREADS, SMEM, stream, b, tin, tout);
+    return launch_kernel<true>(kernel, grid, THREADS, SMEM, stream, b, tin, tout);
 }
 
 // Tile shapes with a TMA kernel (the only ones pass_tma_supported accepts): widths 2 .. 16

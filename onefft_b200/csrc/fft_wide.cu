@@ -99,7 +99,8 @@ __device__ __forceinline__ void pair_stages(float2 (&v)[2][16], int j, int c, in
     }
 }
 
-// SWAP: the first pass exchanges re/im on load, the last on store. W: weights (PassArgs::pre, post). X: a
+// SWAP: the first pass exchanges re/im on load, the last on store. W: the first pass multiplies its input by
+// PassArgs::pre (not NULL). X: a
 // pass of a column transform (PassArgs' column fields, as tma_tile; re/im exchanges at run time): the
 // tile of a.in, the column factors, and the first pass with colstore or the last pass writing the
 // column layout.
@@ -134,8 +135,7 @@ __global__ void __launch_bounds__(Wide<LOG_L, LOG_C>::THREADS, LOG_L + LOG_C >= 
         dependent_wait();  // the other threads touch the caller's buffers only after the copy landed
         load(t);
     }
-    const float2 *pre = nullptr, *post = nullptr;
-    if constexpr (W) pre = a.pre, post = a.post;
+    if constexpr (W) dependent_wait();  // every thread reads the caller's weights
     __syncthreads();  // the barrier is initialised before anyone waits on it
     for (; t < tiles; t += gridDim.x, parity ^= 1u) {
         const unsigned col0 = (t & ((1u << log_tiles) - 1)) << LOG_C;
@@ -158,18 +158,35 @@ __global__ void __launch_bounds__(Wide<LOG_L, LOG_C>::THREADS, LOG_L + LOG_C >= 
             wl[0] = pass_twiddle_lane<LOG_L>(a, f, jl);
             wl[1] = MODE == 0 ? pass_twiddle_lane<LOG_L>(a, f + 1, jl) : wl[0];
         }
-        const bool ok = !g_expire_waits && mbar_wait(bar, parity);
         float2 v[2][16];
+        if constexpr (W) {  // the weights first, in the registers of the values they multiply
+            const float2* w = a.pre + col0 + 2 * c + ((unsigned)j << a.log_s);
+            const unsigned step = (unsigned)G::T << a.log_s;
+            if (((uintptr_t)a.pre & 15) == 0) {
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    const float4 x = ld_stream4(w + k * step);
+                    v[0][k] = make_float2(x.x, x.y);
+                    v[1][k] = make_float2(x.z, x.w);
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 16; ++k) v[0][k] = ld_stream(w + k * step), v[1][k] = ld_stream(w + k * step + 1);
+            }
+        }
+        const bool ok = !g_expire_waits && mbar_wait(bar, parity);
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
             const float4 x = *reinterpret_cast<const float4*>(land + (j + G::T * k) * G::C + 2 * c);
-            v[0][k] = make_float2(x.x, x.y);
-            v[1][k] = make_float2(x.z, x.w);
+            if constexpr (W) {
+                v[0][k] = cmul(make_float2(x.x, x.y), v[0][k]);
+                v[1][k] = cmul(make_float2(x.z, x.w), v[1][k]);
+            } else {
+                v[0][k] = make_float2(x.x, x.y);
+                v[1][k] = make_float2(x.z, x.w);
+            }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                if constexpr (W && MODE == 0) {
-                    if (pre) v[i][k] = cmul(v[i][k], __ldg(pre + col0 + 2 * c + i + ((unsigned)(j + G::T * k) << a.log_s)));
-                }
                 if (X ? a.swap_in : SWAP && MODE == 0) v[i][k] = swap_ri(v[i][k]);
             }
         }
@@ -227,12 +244,7 @@ __global__ void __launch_bounds__(Wide<LOG_L, LOG_C>::THREADS, LOG_L + LOG_C >= 
                 const unsigned e = base + ((unsigned)(j + G::T * k) << a.log_s);
                 float2 y[2];
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    y[i] = (X ? a.swap_out : SWAP && MODE == 2) ? swap_ri(v[i][k]) : v[i][k];
-                    if constexpr (W && MODE == 2) {
-                        if (post) y[i] = cmul(y[i], __ldg(post + e + i));
-                    }
-                }
+                for (int i = 0; i < 2; ++i) y[i] = (X ? a.swap_out : SWAP && MODE == 2) ? swap_ri(v[i][k]) : v[i][k];
                 *reinterpret_cast<float4*>(X ? qx + part(k) : a.out + toff + e) = make_float4(y[0].x, y[0].y, y[1].x, y[1].y);
             }
         }
@@ -264,16 +276,31 @@ static cudaError_t launch_wide_w(const PassArgs& a, int batch, cudaStream_t stre
     const int log_tiles = a.log2n - LOG_L - LOG_C;
     const unsigned tiles = (unsigned)batch << log_tiles;
     if ((unsigned)grid > tiles) grid = (int)tiles;
-    return launch_kernel<!W>(kernel, dim3((unsigned)grid), G::THREADS, G::SMEM, stream, a, tin, tiles, log_tiles);
+    return launch_kernel<true>(kernel, dim3((unsigned)grid), G::THREADS, G::SMEM, stream, a, tin, tiles, log_tiles);
+}
+
+// Weights cost a persistent block of one tile an SM more than the small blocks of k_pass_tma: their 16- to
+// 64-byte row pieces arrive by per-thread loads, which nothing overlaps but the tile's own copy. First passes of
+// up to 2^10 values take them (128-byte pieces, loaded while the copy is in flight); longer first passes and all
+// last ones go to k_pass_tma. Wide against k_pass_tma for the weighted pass, us (B200, warm): input weights,
+// 16 x 2^21 299 / 288, 2^22 48.1 / 43.0, 4 x 2^23 424 / 351, 2^24 224 / 190 (2^20, which stays: 32 x 255 / 266);
+// output weights, 64 x 2^19 283 / 238, 32 x 2^20 298 / 268, 16 x 2^21 322 / 290, 2^22 48.5 / 43.4, 2^23 107 / 92,
+// 2^24 221 / 201, 2^28 3392 / 3367.
+constexpr int kWideWeightsLog2 = 10;
+bool pass_wide_weights(int mode, int log_l, const PassArgs& a) {
+    return mode == 0 ? !a.pre || log_l <= kWideWeightsLog2 : mode == 1 || !a.post;
 }
 
 template <int LOG_L, int LOG_C, int MODE>
 static cudaError_t launch_wide_t(const PassArgs& a, int batch, cudaStream_t stream) {
     const bool swap = MODE == 0 ? a.swap_in : a.swap_out;
-    if constexpr (MODE != 1) {
-        if (MODE == 0 ? a.pre != nullptr : a.post != nullptr)
+    if constexpr (MODE == 0 && LOG_L <= kWideWeightsLog2) {
+        if (a.pre)
             return swap ? launch_wide_w<LOG_L, LOG_C, MODE, true, true>(a, batch, stream)
                         : launch_wide_w<LOG_L, LOG_C, MODE, false, true>(a, batch, stream);
+    }
+    if (!pass_wide_weights(MODE, LOG_L, a)) return cudaErrorInvalidValue;
+    if constexpr (MODE != 1) {
         if (swap) return launch_wide_w<LOG_L, LOG_C, MODE, true, false>(a, batch, stream);
     }
     return launch_wide_w<LOG_L, LOG_C, MODE, false, false>(a, batch, stream);

@@ -550,7 +550,10 @@ static cudaError_t plan_enqueue(const onefft_plan *p, const float2 *in, float2 *
     const bool use_tma = p->tma && !p->tc && batch <= 65535 && ((((uintptr_t)in | (uintptr_t)out) & 15) == 0);
     auto run = [&](int mode, int i, const PassArgs &x) {
         const int wide = p->cols[i] & kWideTile, cols = p->cols[i] & ~kWideTile;
-        if (use_tma && wide) return launch_pass_wide(mode, p->len[i], cols, x, (int)batch, s);
+        if (use_tma && wide && pass_wide_weights(mode, p->len[i], x))
+            return launch_pass_wide(mode, p->len[i], cols, x, (int)batch, s);
+        if (use_tma && wide)  // weighted: the widest tile that k_pass_tma has for the length
+            return launch_pass_tma(mode, p->len[i], pass_tma_supported(p->len[i], cols) ? cols : cols - 1, x, (int)batch, s);
         if (use_tma && pass_tma_supported(p->len[i], cols))
             return launch_pass_tma(mode, p->len[i], cols, x, (int)batch, s);
         return p->tc ? launch_pass_tc(mode, p->len[i], x, (int)batch, p->tc, s)

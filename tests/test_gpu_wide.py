@@ -104,3 +104,25 @@ def test_expired_wait_is_reported(ofb, log2n):
     transform(plan, x, out, 1, False)
     want = torch.fft.fft(torch.view_as_complex(x.view(-1, 2)).to(torch.complex128))
     assert float((torch.view_as_complex(out.view(-1, 2)) - want).abs().norm() / want.abs().norm()) < 1e-6
+
+
+@pytest.mark.parametrize("log2n,batch", [(18, 3), (19, 2), (20, 3), (21, 1), (22, 2), (23, 1), (24, 1), (28, 1), (29, 1), (30, 1)])
+@pytest.mark.parametrize("shift", [0, 1])  # offset of the weights in complex values: 1 = not 16-byte aligned
+def test_weights_equal_plain_passes(ofb, log2n, batch, shift):
+    """Both weights at once, aligned and not, where weighted passes split between the wide tiles and
+    k_pass_tma: the bits of the plain passes of the same split; nothing is written past the output."""
+    import torch
+    if shift and log2n > 28:
+        pytest.skip("one case of the sizes that hold tens of gigabytes")
+    n = 1 << log2n
+    splits = {**SPLITS, 29: ((9, 10, 10),), 30: ((10, 10, 10),)}
+    g = torch.Generator(device="cuda").manual_seed(log2n)
+    x = torch.randn(2 * n * batch, device="cuda", generator=g)
+    pre, post = (torch.randn(2 * n + 2 * shift, device="cuda", generator=g)[2 * shift:] for _ in range(2))
+    a, b = (torch.full((2 * n * batch + 4,), 7.0, device="cuda") for _ in range(2))
+    default, plain = ofb.Plan(n), ofb.Plan(n, split=splits[log2n][0], l2_keep=False)
+    for inverse in (False, True):
+        transform(default, x, a, batch, inverse, pre, post)
+        transform(plain, x, b, batch, inverse, pre, post)
+        assert torch.equal(a, b)
+        assert bool((a[-4:] == 7.0).all())
