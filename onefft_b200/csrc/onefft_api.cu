@@ -1309,9 +1309,13 @@ extern "C" int onefft_uneven_execute(onefft_uneven *u, const float *d_in, float 
     // 2^4 .. 2^9, 117 thousand values, 8.2 -> 6.9 us; 2000 of 2^9 .. 2^12 24.7 -> 22.2; 300 of 2^10 ..
     // 2^16 64 -> 52). The line lies between 17 and 117 thousand values.
     cudaError_t e = cudaSuccess;
-    // (A captured stream takes the graph path whatever the size: its launch is refused there.)
+    // (A captured stream takes the graph path whatever the size: its launch is refused there. So does a call
+    // with another device current than the batch's: the graph's node belongs to the batch's device, a
+    // launch goes to the current one, where the batch's tables and counters are not.)
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (u->span > ((size_t)1 << 16) && cudaStreamIsCapturing((cudaStream_t)stream, &cs) == cudaSuccess &&
+    int cur = -1;
+    if (u->span > ((size_t)1 << 16) && cudaGetDevice(&cur) == cudaSuccess && cur == u->device &&
+        cudaStreamIsCapturing((cudaStream_t)stream, &cs) == cudaSuccess &&
         cs == cudaStreamCaptureStatusNone) {
         UnevenArgs args = u->args;
         args.in = (const float2 *)d_in;

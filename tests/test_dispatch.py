@@ -1,0 +1,39 @@
+"""CPU tests of which kernels a call is routed to: the library's host code compiled against a stand-in for
+the CUDA runtime and the kernel launchers (tests/c_api/check_dispatch.cpp), which prints every launch.
+"""
+from __future__ import annotations
+
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def launches(tmp_path_factory):
+    cxx = next((c for c in map(shutil.which, ("c++", "g++")) if c), None)
+    inc = os.path.join(CUDA_HOME, "include")
+    if cxx is None or not os.path.exists(os.path.join(inc, "cuda_runtime.h")):
+        pytest.skip("no C++ compiler or no CUDA runtime headers")
+    csrc = os.path.join(ROOT, "onefft_b200", "csrc")
+    exe = str(tmp_path_factory.mktemp("dispatch") / "check_dispatch")
+    cmd = [cxx, "-std=c++17", "-O1", "-I", os.path.join(ROOT, "include"), "-I", csrc, "-I", inc, "-x", "c++",
+           os.path.join(csrc, "onefft_api.cu"), os.path.join(ROOT, "tests", "c_api", "check_dispatch.cpp"), "-o", exe]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+    def run(*args) -> list[str]:
+        r = subprocess.run([exe, *map(str, args)], capture_output=True, text=True)
+        assert r.returncode == 0, r.stdout + r.stderr
+        return r.stdout.splitlines()
+    return run
+
+
+def test_uneven_batch_runs_on_its_own_device(launches):
+    """A batch made on device 0 runs there whatever device is current, below and beyond the span from which
+    on its kernel is launched directly."""
+    assert launches("uneven_device") == ["graph on device 0", "graph on device 0", "kernel on device 0", "graph on device 0"]
