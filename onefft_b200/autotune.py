@@ -186,15 +186,15 @@ def time_plan(plan, x, y, reps: int, flush) -> float:
     return ts[len(ts) // 2]
 
 
-# ONEFFT_COLS_PIPELINED: the persistent double-buffered one-kernel form of 2^12 and 2^13
+# ONEFFT_COLS_PIPELINED: the persistent one-kernel form of 2^12 and 2^13
 PIPELINED = 15
 
 
 def batched_log_c_candidates(l: int) -> list[int]:
     """Transforms per block (log2) compiled for the one-kernel size 2^l (fft_kernels.cu,
     batched_log_c_supported): the default 4096 / n, half and twice that up to 8192 values; at 2^12
-    also the pipelined form (fft_tma.cu, batched_pipe_supported); 2^13 and 2^14 run pipelined
-    whatever the width (fft_long.cu)."""
+    and 2^13 also the pipelined form (fft_tma.cu, batched_pipe_supported; fft_long.cu). 2^14 has one
+    width to choose; the tuned plan runs its pipelined form (fft_long.cu)."""
     b = max(0, 12 - l)
     out = [c for c in (b - 1, b, b + 1) if c == b or (c >= 0 and l + c <= 13)]
     return out + ([PIPELINED] if l in (12, 13) else [])
@@ -217,7 +217,7 @@ def tune_batched(reps: int = 9) -> dict:
         p0.dev_forward(x.data_ptr(), ref.data_ptr(), batch)
         p0.destroy()
         times = {}
-        for c in batched_log_c_candidates(l):
+        for c in batched_log_c_candidates(l) + ([-1] if l == 14 else []):  # 2^14: the tuned plan is the pipelined form
             plan = ofb.Plan(n, split=(l,), cols=(c,))
             y.fill_(float("nan"))
             plan.dev_forward(x.data_ptr(), y.data_ptr(), batch)
@@ -239,14 +239,14 @@ def tune_batched(reps: int = 9) -> dict:
             times[c] = ts[len(ts) // 2]
         best = min(times, key=times.get)
         out[l] = {"log_c": best, "us": times}
-        label = lambda c: "pipelined" if c == PIPELINED else f"{1 << c}/block"  # noqa: E731
+        label = lambda c: "pipelined" if c in (PIPELINED, -1) else f"{1 << c}/block"  # noqa: E731
         print(f"batched 2^{l} x {batch}: " + ", ".join(f"{label(c)} {t:.1f} us" for c, t in times.items()) +
               f" -> {label(best)}", flush=True)
         del x, ref, y
         torch.cuda.empty_cache()
     table = [-1] * 15
     for l, r in out.items():
-        table[l] = r["log_c"]
+        table[l] = PIPELINED if r["log_c"] < 0 else r["log_c"]
     print("static const int kBatchedTunedLogC[kMaxSingleLog2 + 1] = {" + ", ".join(str(v) for v in table) + "};")
     return out
 

@@ -213,12 +213,17 @@ static const Shape kPlain[] = {
 static_assert(sizeof(kPlain) / sizeof(kPlain[0]) == 30 - 17 + 1, "one shape per size 2^17 .. 2^30");
 static const Shape *plain_shape(int m) { return m < 17 ? nullptr : &kPlain[m - 17]; }
 
+// One kernel, cols[0] = this: a persistent pipelined kernel instead of k_batched (ONEFFT_COLS_PIPELINED in
+// onefft_cuda.h): launch_batched_pipe at 2^12, launch_batched_long at 2^13 and, as the tuned choice only, 2^14.
+constexpr int kPipelinedCols = 15;
+
 // Transforms per block (log2) of the one-kernel sizes 2^4 .. 2^14, from
 // `python -m onefft_b200.autotune --batched` on a B200 (forward, 2^25 values per batch, median of
 // 9): 2048-value tiles up to n = 2^9 and at 2^11 (2^4 87 us against 90 / 96 for 4096 / 8192, 2^5
 // 86 against 94 / 131, 2^6 87 against 96 / 133; 2^7 .. 2^9 and 2^11 by one timer tick, ~2 us),
-// the default 4096 at 2^10 and 2^12; 2^13 / 2^14 have one width. -1 = the default.
-static const int kBatchedTunedLogC[kMaxSingleLog2 + 1] = {-1, -1, -1, -1, 7, 6, 5, 4, 3, 2, 2, 0, 0, 0, 0};
+// the default 4096 at 2^10 and 2^12. 2^13 and 2^14 run pipelined (launch_batched_long: 4096 x 2^13 104 us
+// against 124 with the one width they have, 2048 x 2^14 135 against 153). -1 = the default.
+static const int kBatchedTunedLogC[kMaxSingleLog2 + 1] = {-1, -1, -1, -1, 7, 6, 5, 4, 3, 2, 2, 0, 0, kPipelinedCols, kPipelinedCols};
 
 static Shape tuned_shape(int m) {
     Shape s{};
@@ -231,15 +236,11 @@ static Shape tuned_shape(int m) {
     return kTuned[m - 15];
 }
 
-// One kernel, cols[0] = this: the persistent pipelined kernel (launch_batched_pipe) instead of
-// k_batched at 2^12 (ONEFFT_COLS_PIPELINED in onefft_cuda.h; 2^13 is pipelined whatever the width).
-constexpr int kPipelinedCols = 15;
-
 static bool valid_shape(int m, const Shape &s) {
     if (s.npass == 1)
         return s.len[0] == m && m <= kMaxSingleLog2 &&
                (s.cols[0] == -1 || batched_log_c_supported(m, s.cols[0]) ||
-                (s.cols[0] == kPipelinedCols && (batched_pipe_supported(m) || m == 13)));
+                (s.cols[0] == kPipelinedCols && (batched_pipe_supported(m) || (m == 13 && batched_long_supported(m)))));
     if (s.npass < 2 || s.npass > 3) return false;
     int sum = 0;
     for (int p = 0; p < s.npass; ++p) {
@@ -415,11 +416,13 @@ extern "C" onefft_plan *onefft_plan_create_tiles(size_t n, int npass, const int 
         s.cols[i] = log2_cols ? log2_cols[i] : pass_log_c(log2_len[i]);
     }
     // one kernel: cols[0] is the transforms per block (log2), the tuned one unless given
-    if (npass == 1 && (!log2_cols || log2_cols[0] == -1)) s.cols[0] = m <= kMaxSingleLog2 ? tuned_shape(m).cols[0] : -1;
+    const bool tuned_cols = npass == 1 && (!log2_cols || log2_cols[0] == -1);
+    if (tuned_cols) s.cols[0] = -1;
     if (!valid_shape(m, s)) {
         set_error(ONEFFT_ERR_ARG, "invalid pass split for n=%zu", n);
         return nullptr;
     }
+    if (tuned_cols) s.cols[0] = tuned_shape(m).cols[0];
     return plan_build(n, m, s);
 }
 
@@ -524,13 +527,13 @@ static cudaError_t plan_enqueue(const onefft_plan *p, const float2 *in, float2 *
     if (p->npass == 1) {
         g_launches.fetch_add(1);
         if (p->tc) return launch_single_kernel_tc(p->log2n, in, out, batch, p->stw[0], inverse, p->tc, s);
-        // 2^13 and 2^14 through bulk copies where the input allows them (k_batched otherwise: 5-20 %
-        // slower from 150 transforms on, a tick slower below; the same bits)
-        if (batched_long_supported(p->log2n) && !((uintptr_t)in & 15))
-            return launch_batched_long(p->log2n, in, out, batch, p->stw[0], inverse, p->err, s, pre, post);
         if (p->cols[0] == kPipelinedCols) {
-            // bulk copies need 16-byte aligned transforms; weighted calls use k_batched's weights
-            if (!pre && !post && !((uintptr_t)in & 15))
+            // bulk copies need 16-byte aligned transforms (k_batched otherwise: the same bits); weighted calls
+            // of 2^12 use k_batched's weights
+            const bool aligned = !((uintptr_t)in & 15);
+            if (aligned && batched_long_supported(p->log2n))
+                return launch_batched_long(p->log2n, in, out, batch, p->stw[0], inverse, p->err, s, pre, post);
+            if (aligned && !pre && !post)
                 return launch_batched_pipe(p->log2n, in, out, batch, p->stw[0], inverse, p->err, s);
             return launch_single_kernel(p->log2n, in, out, batch, p->stw[0], inverse, s, pre, post, -1);
         }

@@ -37,3 +37,21 @@ def test_uneven_batch_runs_on_its_own_device(launches):
     """A batch made on device 0 runs there whatever device is current, below and beyond the span from which
     on its kernel is launched directly."""
     assert launches("uneven_device") == ["graph on device 0", "graph on device 0", "kernel on device 0", "graph on device 0"]
+
+
+@pytest.mark.parametrize("log2n,width,kernel", [(13, None, "long"), (13, -1, "long"), (13, 15, "long"), (13, 0, "batched"),
+                                                (14, None, "long"), (14, -1, "long"), (14, 0, "batched"), (12, None, "batched"),
+                                                (12, 15, "pipe"), (12, 0, "batched"), (12, 1, "batched"), (14, 15, None), (13, 1, None)])
+@pytest.mark.parametrize("shift", [0, 1])  # offset of the buffers in complex values: 1 = not 16-byte aligned
+def test_explicit_width_selects_its_kernel(launches, log2n, width, kernel, shift):
+    """onefft_plan_create_tiles with one kernel: a width given runs k_batched with it, the pipelined choice
+    and the tuned one (NULL or -1) the pipelined kernels where the input is aligned."""
+    got = launches("widths", log2n, shift, *([] if width is None else [width]))
+    if kernel is None:
+        assert got == [f"invalid pass split for n={1 << log2n}"]
+        return
+    assert len(got) == 1
+    words = got[0].split()
+    assert words[0] == (kernel if shift == 0 else "batched")
+    if kernel == "batched" and width is not None and width >= 0:
+        assert words[2] == str(width)  # (the stand-in prints the width as the mode)
