@@ -190,8 +190,7 @@ static_assert(sizeof(kTuned) / sizeof(kTuned[0]) == 30 - 15 + 1, "one shape per 
 // against 29, 512 86 against 100).
 constexpr int kClusterBatch = 360;
 
-// The passes of calls whose buffers do not allow bulk tensor copies (not 16-byte aligned, or more
-// than 65535 transforms), 2^17 .. 2^30: per-thread loads run the long columns of the shapes above in
+// The passes of calls whose buffers do not allow bulk tensor copies (not 16-byte aligned), 2^17 .. 2^30: per-thread loads run the long columns of the shapes above in
 // blocks of 1024 threads, one per SM (2^24 in (12,12) 217 us against 185 in (8,8,8), 2^23 107
 // against 91, 2^28 3574 against 3438).
 static const Shape kPlain[] = {
@@ -550,7 +549,16 @@ static cudaError_t plan_enqueue(const onefft_plan *p, const float2 *in, float2 *
     a.pre = pre;
     a.post = post;
     // pass i through its TMA kernel where the plan asks for it and the shape and buffers allow
-    const bool use_tma = p->tma && !p->tc && batch <= 65535 && ((((uintptr_t)in | (uintptr_t)out) & 15) == 0);
+    const bool use_tma = p->tma && !p->tc && ((((uintptr_t)in | (uintptr_t)out) & 15) == 0);
+    // these kernels take up to 65535 transforms a launch
+    if (use_tma && batch > 65535) {
+        for (long long b = 0; b < batch; b += 65535) {
+            const cudaError_t e = plan_enqueue(p, in + (b << p->log2n), out + (b << p->log2n), std::min(batch - b, 65535ll),
+                                               inverse, s, pre, post);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
     auto run = [&](int mode, int i, const PassArgs &x) {
         const int wide = p->cols[i] & kWideTile, cols = p->cols[i] & ~kWideTile;
         if (use_tma && wide && pass_wide_weights(mode, p->len[i], x))

@@ -55,3 +55,25 @@ def test_explicit_width_selects_its_kernel(launches, log2n, width, kernel, shift
     assert words[0] == (kernel if shift == 0 else "batched")
     if kernel == "batched" and width is not None and width >= 0:
         assert words[2] == str(width)  # (the stand-in prints the width as the mode)
+
+
+@pytest.mark.parametrize("log2n", [15, 16, 17, 20])
+def test_batches_beyond_a_launch_keep_their_kernels(launches, log2n):
+    """Aligned batches of more than 65535 transforms go through the same kernels as smaller ones, in slices
+    (so a transform's bits do not depend on its batch); unaligned ones are one call of the plain passes."""
+    small = [line.split() for line in launches("default", log2n, 60000, 0)]
+    for batch, sizes in ((65535, [65535]), (65536, [65535, 1]), (131471, [65535, 65535, 401])):
+        got = [line.split() for line in launches("default", log2n, batch, 0)]
+        first = 0
+        for size in sizes:
+            # the last slice of 2^15 may be short of the cluster kernel's line
+            want = [line.split() for line in launches("default", log2n, size, 0)]
+            for words in want:
+                mine = got.pop(0)
+                assert mine[:7] == words[:7]
+                assert int(mine[8]) - int(words[8]) == int(mine[10]) - int(words[10]) == first << log2n
+            if size == 65535:
+                assert [w[:5] for w in want] == [w[:5] for w in small]
+            first += size
+        assert got == []
+    assert {line.split()[0] for line in launches("default", log2n, 65536, 1)} == {"pass"}

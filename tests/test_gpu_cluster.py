@@ -77,3 +77,19 @@ def test_many_rounds_forward(ofb):
         torch.cuda.synchronize()
         default.check()
         assert torch.equal(out, want)
+
+
+def test_more_transforms_than_a_launch_takes(ofb):
+    """65538 transforms (17 GB a buffer): the ones around the slice's end have the bits of a call of their own."""
+    import torch
+    batch = 65538
+    x = torch.empty(2 * N * batch, device="cuda").normal_(generator=torch.Generator(device="cuda").manual_seed(3))
+    out = torch.full_like(x, 7.0)
+    plan = ofb.Plan(N)
+    plan.dev_forward(x.data_ptr(), out.data_ptr(), batch)
+    for first in (0, batch - 6):
+        want = torch.empty(2 * N * 6, device="cuda")
+        plan.dev_forward(x.data_ptr() + 8 * N * first, want.data_ptr(), 6)
+        torch.cuda.synchronize()
+        plan.check()
+        assert torch.equal(out[2 * N * first:2 * N * (first + 6)], want)
