@@ -23,13 +23,14 @@ cudaError_t set_expire_waits_cluster(int on) {
 // The next transform's copy is issued when a block has read its rows, half a transform ahead.
 // Two cluster barriers a transform: one says that every landing buffer is free (arrived at early, waited
 // for late), one that the rows have arrived. The first arrival releases this thread's reads of its
-// landing buffer to the peers that overwrite it, and nothing else (cluster_arrive_shared). A block's columns are the same for every
-// transform it takes, so the inter-pass factors are computed once per launch.
+// landing buffer to the peers that overwrite it, and nothing else (cluster_arrive_shared). A block's
+// columns are the same for every transform it takes, so the inter-pass factors are computed once per
+// launch.
 //
-// Measured on a B200, warm, against the two passes: 2000 x 2^15 293 us against 331, 512 x 2^15 86
-// against 93 (two trips of 268 MB through HBM at the board's power limit). What bounds it: a block's
-// load, two transforms and exchanges follow each other (one block an SM, 10.4 us a transform), so it needs
-// many transforms per cluster: 160 x 2^15 (three rounds of 72 clusters) 40 us against 29. The same
+// Measured on a B200, warm, against the two passes: 2000 x 2^15 293 us against 351, 512 x 2^15 86
+// against 95 (two trips of 268 MB through HBM at the board's power limit). What bounds it: a block's
+// load, two transforms and exchanges follow each other (one block an SM, 10.4 us a transform), so it
+// needs many transforms per cluster: 160 x 2^15 (three rounds of 72 clusters) 40 us against 29. The same
 // with four blocks for 2^16 was slower than two passes (1000 transforms 405 us against 372; 33 clusters
 // fit the device, and three quarters of the values cross blocks) and is not built.
 template <int Q>
@@ -76,7 +77,6 @@ __global__ void __cluster_dims__(Q, 1, 1) __launch_bounds__(512, 1)
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int stride = (int)gridDim.x / Q;
     long long t = blockIdx.x / Q;  // the same for the whole cluster; the grid has no more clusters than transforms
-    dependent_launch();
     auto load = [&](long long b) {
         mbar_expect_tx(bar, 131072u);
         tma_load_4d(cl_smem, &tin, (int)rank * 64, 0, 0, (int)b, bar);

@@ -15,17 +15,19 @@ namespace ofb {
 
 // ---- programmatic dependent launch ---------------------------------------------------------------
 //
-// Every transform kernel starts with dependent_launch(). In a grid of at least kDependentBlocks
-// blocks it lets the stream's next kernel be scheduled once all blocks of this one run, so that
-// its first blocks fill the slots this kernel's last blocks leave free; smaller grids only release
-// it as they finish. (The early blocks of the next kernel go to whichever SMs have room: behind
-// a grid that fills few slots they crowd on some SMs. Released early from any grid, 8 x 2^16 took
-// 14.3 us instead of 7.4 and 2^20 20.0 us instead of 12.7; a floor of 296 or 592 blocks left other
-// sizes slow (5 x 2^17 19.5 us instead of 9.4); 1184, 8 blocks an SM, none. Never releasing early
-// costs 1-2 % at 2^22 .. 2^24.)
+// Transform kernels with a block per tile (k_tiny, k_batched, k_pass, k_pass_tma) start with
+// dependent_launch(). In a grid of at least kDependentBlocks blocks it lets the stream's next kernel
+// be scheduled once all blocks of this one run, so that its first blocks fill the slots this kernel's
+// last blocks leave free; smaller grids only release it as they finish. (The early blocks of the next
+// kernel go to whichever SMs have room: behind a grid that fills few slots they crowd on some SMs.
+// Released early from any grid, 8 x 2^16 took 14.3 us instead of 7.4 and 2^20 20.0 us instead of 12.7; a
+// floor of 296 or 592 blocks left other sizes slow (5 x 2^17 19.5 us instead of 9.4); 1184, 8 blocks an
+// SM, none. Never releasing early costs 1-2 % at 2^22 .. 2^24.) The persistent kernels never have that
+// many blocks and do not call it.
 // dependent_wait() returns when the previous kernel has completed and its writes are visible; it
 // comes before the first access to the caller's buffers (plan tables, written at plan creation, may
-// be read earlier). Without a predecessor that allows the overlap both do nothing.
+// be read earlier), whose loads go through L2 (ld_stream, fft_tiles.cuh). Without a predecessor that
+// allows the overlap both do nothing.
 constexpr unsigned kDependentBlocks = 1184;
 __device__ __forceinline__ void dependent_launch() {
     if (gridDim.x >= kDependentBlocks || gridDim.x * gridDim.y >= kDependentBlocks)

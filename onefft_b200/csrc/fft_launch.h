@@ -25,8 +25,8 @@ inline cudaError_t smem_limit(const void* kernel, int bytes, std::atomic<unsigne
 }
 
 // Launches a kernel that may start while the stream's previous kernel is still running
-// (programmatic dependent launch): the kernel calls dependent_launch() first and dependent_wait()
-// before it touches the caller's buffers (fft_device.cuh). What a launch, its block scheduling and a
+// (programmatic dependent launch): the kernel calls dependent_wait() before it touches the caller's buffers
+// (fft_device.cuh). What a launch, its block scheduling and a
 // kernel's prologue take (1-3 us) then no longer lies between two kernels of a stream. Measured on a
 // B200, calls back to back: one 2^20 transform (two kernels) 16.4 -> 12.7 us, 2^17 10.3 -> 6.1 us,
 // 2^22 41.8 -> 35.1 us, 2^24 139 -> 132 us, 16 x 2^15 12.3 -> 7.1 us, 100003 x 64 20.9 -> 18.5 us.

@@ -111,7 +111,6 @@ __global__ void __launch_bounds__(256, B == 2 ? 2 : 1)
     auto* ex = reinterpret_cast<typename Lanes<B>::T*>(long_smem + G::EX_OFF);
     uint64_t* bar = reinterpret_cast<uint64_t*>(long_smem + G::BAR_OFF);
     const int j = threadIdx.x;
-    dependent_launch();
     long long b = blockIdx.x;
     unsigned parity = 0;
     if (j == 0) {

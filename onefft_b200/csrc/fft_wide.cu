@@ -113,7 +113,6 @@ __global__ void __launch_bounds__(Wide<LOG_L, LOG_C>::THREADS, LOG_L + LOG_C >= 
     float2* ex = reinterpret_cast<float2*>(wide_smem + G::EX_OFF);
     uint64_t* bar = reinterpret_cast<uint64_t*>(wide_smem + G::BAR_OFF);
     const int tid = threadIdx.x;
-    dependent_launch();
     if (smem_u32(wide_smem) & 127) {  // bulk tensor copies need a 128-byte aligned destination
         if (tid == 0) *(volatile unsigned*)a.err = 2u;
         return;
