@@ -35,7 +35,10 @@ extern "C" {
 /* ---- batched transforms on device memory ------------------------------------------------------
  * Counterpart of calling OneFFT's onefft_plan_forward/_inverse (src/onefft.c:1138-1140) `batch`
  * times on consecutive transforms: transform b reads d_in + 2 n b and writes d_out + 2 n b.
- * d_in and d_out are device pointers aligned to 8 bytes (one complex64) that do not overlap. */
+ * d_in and d_out are device pointers aligned to 8 bytes (one complex64) that do not overlap. A
+ * transform's result does not depend on the batch it is in. At 2^17, 2^19, 2^20, 2^22 .. 2^24 and
+ * 2^28 .. 2^30 buffers that are not both 16-byte aligned take another pass split, with the same error
+ * but other rounding. */
 ONEFFT_API int onefft_dev_forward_batched(const onefft_plan *plan, const float *d_in, float *d_out, size_t batch, void *stream);
 ONEFFT_API int onefft_dev_inverse_batched(const onefft_plan *plan, const float *d_in, float *d_out, size_t batch, void *stream);
 
@@ -140,9 +143,9 @@ ONEFFT_API int onefft_plan_passes(const onefft_plan *plan, int *log2_len);
  * plan per size (src/onefft.c:1138-1140): many transforms of different power-of-two sizes packed
  * in one buffer, run by ONE persistent kernel launch that pulls work from a device queue and
  * leaves its counters reset: a CUDA graph built by onefft_uneven_create() and replayed by each
- * execute, or, beyond 2^16 values, a plain launch of the same kernel. Transform i has size 2^log2n (0 <= log2n <= 16), starts at complex offset
- * `offset` of both buffers, and runs forward (inverse = 0) or inverse (inverse = 1). Transforms
- * must not overlap each other. */
+ * execute, or, beyond 2^16 values and with the batch's device current, a launch of the same kernel.
+ * Transform i has size 2^log2n (0 <= log2n <= 16), starts at complex offset `offset` of both buffers,
+ * and runs forward (inverse = 0) or inverse (inverse = 1). Transforms must not overlap each other. */
 typedef struct onefft_desc {
     int32_t log2n;
     int32_t inverse;

@@ -131,9 +131,10 @@ struct onefft_plan {
 // where the buffers allow bulk tensor copies.
 constexpr int kWideTile = 16;
 
-// How a size runs: number of passes, their lengths and tile widths. The table below is the
-// tuned choice per log2 n (onefft_b200/autotune.py measures the candidates on the device and
-// prints this table); sizes up to 2^14 run as one kernel.
+// How a size runs: number of passes, their lengths and tile widths. The tables below are the tuned
+// choices per log2 n; sizes up to 2^14 run as one kernel. (onefft_b200/autotune.py times the shapes of
+// k_pass and k_pass_tma, which onefft_plan_create_tiles can make, and prints the fastest; the wide tiles
+// were timed by hand, and plans with them come from these tables only.)
 struct Shape {
     int npass;
     int len[3];
@@ -147,19 +148,20 @@ struct Shape {
 // Shapes by size: {npass, {log2 lengths}, {log2 tile widths}, l2_keep, chunk, tma}; W(c): the wide-tile
 // kernel with 2^c columns (fft_wide.cu), else k_pass_tma (tma) or k_pass. Timed on a B200 with calls
 // back to back on three buffer pairs in turn, warm for 0.3 s (the clock then sits where the board's
-// power limit leaves it), single transforms and batches up to 2^26 values; one shape per size,
-// so that a transform's bits do not depend on its batch. us, this table against the shapes before it
-// (all with dependent launches), at batch 1 / a small batch / a large one:
-//   2^17 (10,7)     5.6 / 36.0 (32) / 262 (256)  ->  6.7 / 27.4 / 199
-//   2^18 (10,8)     6.6 / 33.8 (16) / 248 (128)  ->  8.0 / 28.8 / 204
-//   2^19 (8,11)     9.0 / 43.5 (8)  / 315 (64)   ->  9.2 / 29.0 / 212
-//   2^20 (12,8)    13.2 / 28.4 (3)  / 258 (32)   -> 11.0 / 26.3 / 217
-//   2^21 (11,10)   21.7 / 53.0 (3)  / 272 (16)   -> 19.9 / 47.6 / 223
-//   2^22 (8,7,7)   35.4 / 99.9 (3)  / 281 (8)    -> 36.3 / 95.9 / 231
-//   2^23 (8,8,7)   62.6 /             288 (4)    -> 67.5 /        240
-//   2^24 (8,8,8)   143  /             281 (2)    -> 132  /        254
-//   2^28 (10,10,8) 2702 -> (9,9,10) 2408;  2^29 (10,10,9) 5534 -> (9,10,10) 5162;
-//   2^30 (10,11,9) 11499 -> (10,10,10) 10571
+// power limit leaves it), single transforms and batches up to 2^26 values; one shape per size, so
+// that a transform's bits do not depend on its batch (those of calls that do not allow bulk copies are
+// kPlain's). us, the shapes before it / this table (all with dependent launches), at batch 1 / a small
+// batch / a large one:
+//   2^17 (10,7)     5.5 / 33.5 (32) / 251 (256)  ->  6.6 / 25.9 / 194
+//   2^18 (10,8)     6.7 / 30.9 (16) / 242 (128)  ->  8.2 / 28.7 / 208
+//   2^19 (8,11)     8.6 / 41.3 (8)  / 307 (64)   ->  9.1 / 28.4 / 215
+//   2^20 (12,8)    12.4 / 27.0 (3)  / 257 (32)   -> 10.9 / 25.4 / 218
+//   2^21 (11,10)   19.6 / 50.9 (3)  / 266 (16)   -> 18.7 / 46.7 / 224
+//   2^22 (8,7,7)   34.2 / 100  (3)  / 281 (8)    -> 35.5 / 94.7 / 231
+//   2^23 (8,8,7)   62.2 / 143  (2)  / 289 (4)    -> 68.8 / 128  / 247
+//   2^24 (8,8,8)   142  /             289 (2)    -> 134  /        263
+//   2^28 (10,10,8) 2735 -> (9,9,10) 2533;  2^29 (10,10,9) 5675 -> (9,10,10) 5373;
+//   2^30 (10,11,9) 11858 -> (10,10,10) 11058
 // 2^15, 2^16 and 2^25 .. 2^27 keep k_pass_tma. No wide shape was faster at 2^15, 2^16 (in (8,8), also
 // the split of the uneven batch's in-block passes, which stay bit-identical to this path) and 2^25.
 // At 2^26 and 2^27 wide shapes gain 1-2 % where the power limit holds the clock down (2^27 1192 .. 1213 us
@@ -186,8 +188,8 @@ static const Shape kTuned[] = {
 static_assert(sizeof(kTuned) / sizeof(kTuned[0]) == 30 - 15 + 1, "one shape per size 2^15 .. 2^30");
 
 // From this many transforms of 2^15 the cluster kernel (fft_cluster.cu; the same bits) is faster than
-// the two passes: five rounds of the 72 clusters a B200 holds (300 transforms 55 us in both, 160 40
-// against 29, 512 86 against 100).
+// the two passes: five rounds of the 72 clusters a B200 holds. Passes / cluster, us: 160 28.6 / 40.1, 288
+// 52.8 / 53.6, 324 59.8 / 64.4, 360 67.2 / 64.4, 400 75.5 / 74.9, 512 94.9 / 85.5, 1000 178 / 158.
 constexpr int kClusterBatch = 360;
 
 // The passes of calls whose buffers do not allow bulk tensor copies (not 16-byte aligned), 2^17 .. 2^30: per-thread loads run the long columns of the shapes above in
