@@ -121,3 +121,33 @@ def test_consumers_of_large_grids(ofb, producer, log2n, kind):
     bits(torch, lambda: (x.clone(), torch.zeros_like(x)), calls)
     first.check()
     assert second.status() == 0
+
+
+@pytest.mark.parametrize("log2n", [7, 8])
+@pytest.mark.parametrize("extra", [-1, 0, 5])  # transforms beyond the 6.3 million values from which on L1 serves
+@pytest.mark.parametrize("shift", [0, 1, 2])
+def test_large_batches_through_l1(ofb, log2n, extra, shift):
+    """2^7 and 2^8 at the line of the ordinary launch with cached loads (csrc/fft_kernels.cu): the bits of
+    two calls below it, nothing written past the batch, and chains as above."""
+    import torch
+    n, batch = 1 << log2n, ((3 << 21) >> log2n) + extra
+    values = batch << log2n
+    plan = ofb.Plan(n)
+    s = torch.cuda.current_stream().cuda_stream
+    x = normal(torch, values + shift, log2n)
+    a, b = (torch.full((2 * (values + shift + 4),), 7.0, device="cuda") for _ in range(2))
+    px, pa, pb = (t.data_ptr() + 8 * shift for t in (x, a, b))
+    half = batch // 2
+    for call in (plan.dev_forward, plan.dev_inverse):
+        call(px, pa, batch, s)
+        call(px, pb, half, s)
+        call(px + 8 * n * half, pb + 8 * n * half, batch - half, s)
+        torch.cuda.synchronize()
+        assert torch.equal(a, b)
+        assert bool((a[2 * (values + shift):] == 7.0).all())
+    calls = []
+    for _ in range(4):
+        calls.append(lambda u, v: plan.dev_forward(u.data_ptr() + 8 * shift, v.data_ptr() + 8 * shift, batch, s))
+        calls.append(lambda u, v: plan.dev_inverse(v.data_ptr() + 8 * shift, u.data_ptr() + 8 * shift, half, s))
+    bits(torch, lambda: (x.clone(), torch.zeros_like(x)), calls)
+    plan.check()
